@@ -299,7 +299,9 @@ inline void bind_p2(const Ctx &ctx) {
     if (b.size() == p2::N_PARAMS && memcmp(b.data(), ctx.p2, sizeof(ctx.p2)) == 0) return;
     CK(cudaSetDevice(ctx.device));
     CK(cudaDeviceSynchronize());  // kernels of the previous constants finish first
-    CK(cudaMemcpyToSymbol(c_p2, ctx.p2, sizeof(ctx.p2)));
+    uint64_t table[p2::N_DEVICE];
+    p2::device_table(ctx.p2, table);
+    CK(cudaMemcpyToSymbol(c_p2, table, sizeof(table)));
     b.assign(ctx.p2, ctx.p2 + p2::N_PARAMS);
 }
 
