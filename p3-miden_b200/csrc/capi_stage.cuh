@@ -38,7 +38,9 @@ P3G_API int p3g_ctx_create(int device, const uint64_t *poseidon2_params130, p3g_
         p3g::bind_p2(x->c);
         x->c.make_pool();
         x->c.enable_cache(8ull << 30);  // up to 64 GB of large buffers kept between proofs
+        x->c.init_hash();
     } catch (const p3g::CudaError &e) {
+        x->c.release();
         delete x;
         return e.status;
     }

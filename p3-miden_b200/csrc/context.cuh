@@ -18,6 +18,7 @@
 #include "merkle.cuh"
 #include "lde.cuh"
 #include "ntt.cuh"
+#include "p2tc.cuh"
 #include "poseidon2.cuh"
 
 namespace p3g {
@@ -148,6 +149,22 @@ struct Ctx {
     // on this context (0: the default, 500)
     uint64_t air_chunk_nodes = 0;
 
+    // Tables of the tensor-core permutation (p2tc.cuh) for this context's
+    // constants, and the word in host memory its kernels set when a wait gave
+    // up (checked by sync). No table: every hash runs on p2_permute_dev.
+    DBuf hash_table;
+    uint32_t *hash_err = nullptr;
+    void init_hash() {
+        std::vector<uint8_t> img;
+        if (!p2t::build_tables(p2, img)) return;
+        std::vector<uint64_t> words(img.size() / 8);
+        memcpy(words.data(), img.data(), img.size());
+        CK(cudaHostAlloc((void **)&hash_err, 64, cudaHostAllocPortable | cudaHostAllocMapped));
+        *hash_err = 0;
+        hash_table = upload(words);
+    }
+    p2t::Args hash_args() const { return p2t::Args{(const uint8_t *)hash_table.p, hash_err}; }
+
     // This context's own stream-ordered memory pool. Buffers freed by one
     // context are reused only by that context, so two contexts driving the
     // same device (server workers) never wait on each other's frees, and the
@@ -184,6 +201,7 @@ struct Ctx {
         if (copy_stream) cudaStreamSynchronize(copy_stream);
         tw.clear();
         ws.release();
+        hash_table.release();
         if (bc) {
             bc->clear();
             bc->alive = false;
@@ -192,6 +210,8 @@ struct Ctx {
         if (stream) cudaStreamSynchronize(stream);
         if (pinned) cudaFreeHost(pinned);
         pinned = nullptr;
+        if (hash_err) cudaFreeHost(hash_err);
+        hash_err = nullptr;
         if (lde_stream) cudaStreamDestroy(lde_stream);
         if (copy_stream) cudaStreamDestroy(copy_stream);
         if (stream) cudaStreamDestroy(stream);
@@ -248,7 +268,13 @@ struct Ctx {
     void d2h(uint64_t *dst, const uint64_t *src, size_t words) {
         if (words) CK(cudaMemcpyAsync(dst, src, words * 8, cudaMemcpyDeviceToHost, stream));
     }
-    void sync() { CK(cudaStreamSynchronize(stream)); }
+    void sync() {
+        CK(cudaStreamSynchronize(stream));
+        if (hash_err && *(volatile uint32_t *)hash_err) {
+            *hash_err = 0;
+            throw CudaError{ERR_TIMEOUT, "hash kernel: a tensor-core wait ran out"};
+        }
+    }
     // upload a small host vector to a fresh device buffer
     DBuf upload(const std::vector<uint64_t> &v) {
         DBuf b = alloc(v.size());
@@ -579,14 +605,49 @@ struct Tree {
     uint64_t layer_off(uint32_t l) const { return 2 * H - 2 * (H >> l); }
 };
 
-// Leaf sponge of one height class of n leaves: one thread per leaf, or one
-// 16-lane group per leaf when the class is small (latency-bound).
+// CTAs of a p2tc.cuh kernel over n_blocks blocks of 128 states of `perms`
+// permutations each: as many groups per CTA as fill the SMs in equal rounds,
+// and enough rounds per CTA (8 permutations per thread) that loading the
+// tables (about 3 us) does not count. One CTA fills an SM; a CTA ends after
+// its rounds, so that other streams' kernels get SMs in between.
+inline merkle::TcShape tc_shape(Ctx &ctx, uint64_t n_blocks, uint64_t perms, unsigned &grid) {
+    int sms = 148;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+    const uint64_t n = (uint64_t)sms;
+    const uint64_t rounds = (n_blocks + n * p2t::kGroups - 1) / (n * p2t::kGroups);
+    merkle::TcShape sh{n_blocks, 1, 1};
+    sh.active = (uint32_t)((n_blocks + n * rounds - 1) / (n * rounds));
+    sh.iters = (uint32_t)std::min<uint64_t>(rounds, perms >= 8 ? 1 : 8 / std::max<uint64_t>(1, perms));
+    grid = (unsigned)((n_blocks + (uint64_t)sh.active * sh.iters - 1) / ((uint64_t)sh.active * sh.iters));
+    return sh;
+}
+template <typename K, typename... Args>
+inline void launch_tc(Ctx &ctx, std::atomic<uint64_t> &attr_done, K kernel, uint64_t n, uint64_t perms, Args... args) {
+    unsigned grid = 1;
+    const merkle::TcShape sh = tc_shape(ctx, n / 128, perms, grid);
+    smem_attr_once(attr_done, kernel, p2t::kSmemBytes);
+    kernel<<<grid, p2t::kThreads, p2t::kSmemBytes, ctx.stream>>>(args..., ctx.hash_args(), sh);
+    CK(cudaGetLastError());
+    ctx.launches++;
+}
+
+// Leaf sponge of one height class of n leaves: one 16-lane group per leaf
+// when the class is small (latency-bound), the tensor-core permutation when
+// it is large, one thread per leaf between.
+constexpr uint64_t kTcLeaves = 1ull << 15;
 inline void launch_leaf_class(Ctx &ctx, const merkle::ClassArgs &a, uint64_t n) {
     const unsigned coop_blocks = (unsigned)((n * 16 + 127) / 128), blocks = (unsigned)((n + 127) / 128);
     if (a.cm && a.n_mats != 1) throw CudaError{ERR_INVALID, "column-major copy of a multi-matrix class"};
     if (n <= merkle::kCoopLeaves) {
         if (a.cm) merkle::leaf_class_coop_kernel<true><<<coop_blocks, 128, 0, ctx.stream>>>(a);
         else merkle::leaf_class_coop_kernel<false><<<coop_blocks, 128, 0, ctx.stream>>>(a);
+    } else if (n >= kTcLeaves && ctx.hash_table.p) {
+        uint64_t perms = 0;
+        for (int m = 0; m < a.n_mats; m++) perms += (a.width[m] + 7) / 8;
+        static std::atomic<uint64_t> attr_cm{0}, attr{0};
+        if (a.cm) launch_tc(ctx, attr_cm, merkle::leaf_class_tc_kernel<true>, n, perms, a);
+        else launch_tc(ctx, attr, merkle::leaf_class_tc_kernel<false>, n, perms, a);
+        return;
     } else {
         if (a.cm) merkle::leaf_class_kernel<true><<<blocks, 128, 0, ctx.stream>>>(a);
         else merkle::leaf_class_kernel<false><<<blocks, 128, 0, ctx.stream>>>(a);
@@ -601,9 +662,13 @@ inline void launch_leaf_class(Ctx &ctx, const merkle::ClassArgs &a, uint64_t n) 
 // per launch (a block keeps at least a warp's worth of parents per level);
 // levels above 128 parents run one 16-lane group per parent, one launch per
 // level; the last levels (at most 128 parents) run in one cluster launch.
-constexpr uint64_t kWideParents = 8192;
+constexpr uint64_t kWideParents = 8192, kTcParents = 1ull << 16;
 inline void compress_layers(Ctx &ctx, Tree &t) {
     uint32_t l = 0;
+    for (; ctx.hash_table.p && l < t.depth && (t.H >> (l + 1)) >= kTcParents; l++) {
+        static std::atomic<uint64_t> attr{0};
+        launch_tc(ctx, attr, merkle::compress_level_tc_kernel, t.H >> (l + 1), 1, t.layers.p, t.H, l);
+    }
     while (l < t.depth && (t.H >> (l + 1)) >= kWideParents) {
         const uint64_t n_parents = t.H >> (l + 1);
         const uint32_t blk = 256;

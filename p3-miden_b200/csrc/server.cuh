@@ -95,6 +95,7 @@ class Server {
             uint64_t share = hbm_budget / n_workers;
             CK(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &share));
             memcpy(c->p2, p2, sizeof(c->p2));
+            c->init_hash();
             ctxs_.push_back(std::move(c));
         }
         bind_p2(*ctxs_[0]);
