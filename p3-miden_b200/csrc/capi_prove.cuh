@@ -329,26 +329,20 @@ P3G_API int p3g_lmcs_prove_batch(p3g_ctx *x, const p3g_tree *t, const uint64_t *
         if (i && indices[i] <= indices[i - 1]) return p3g::ERR_INVALID;
     }
     P3G_TRY(x, {
+        CK(cudaSetDevice(x->c.device));
         std::vector<uint64_t> idx(indices, indices + n);
         p3g::OpeningPlan p;
         p3g::plan_openings(t->t, idx, p);
         uint64_t nf = 0;
         for (auto &r : p.rows) nf += r.padded;
         if (nf > *n_fields || p.sibs.size() > *n_commits) throw p3g::CudaError{p3g::ERR_INVALID, "output buffers too small"};
-        uint64_t of = 0, oc = 0;
-        for (auto &r : p.rows) {
-            CK(cudaMemcpyAsync(fields_out + of, r.src, r.len * 8, cudaMemcpyDeviceToHost, x->c.stream));
-            x->c.sync();
-            for (uint64_t k = r.len; k < r.padded; k++) fields_out[of + k] = 0;
-            of += r.padded;
-        }
-        for (auto *s : p.sibs) {
-            CK(cudaMemcpyAsync(commits_out + 4 * oc, s, 32, cudaMemcpyDeviceToHost, x->c.stream));
-            oc++;
-        }
-        x->c.sync();
-        *n_fields = of;
-        *n_commits = oc;
+        std::vector<p3g::Seg> rows, sibs;
+        for (auto &r : p.rows) rows.push_back({r.src, r.len, 0, r.padded});
+        for (auto *d : p.sibs) sibs.push_back({d, 4, 0, 4});
+        p3g::gather_to_host(x->c, rows, fields_out, t->t.device);
+        p3g::gather_to_host(x->c, sibs, commits_out, t->t.device);
+        *n_fields = nf;
+        *n_commits = p.sibs.size();
     })
 }
 

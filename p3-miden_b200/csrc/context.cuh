@@ -599,6 +599,7 @@ struct Tree {
     uint32_t depth = 0;
     uint64_t H = 0;
     uint32_t alignment = 1;
+    int device = 0;
     std::vector<Mat> mats;
     Mat salt{nullptr, 0, 0};  // hiding LMCS: H x SALT per-leaf salt, absorbed last (borrowed)
     uint64_t root[4] = {0, 0, 0, 0};
@@ -740,6 +741,7 @@ inline void build_zero_tree(Ctx &ctx, Tree &t, const std::vector<Mat> &mats, uin
 inline void build_tree(Ctx &ctx, Tree &t, const std::vector<Mat> &mats_in, uint32_t alignment,
                        const Mat *salt = nullptr) {
     t.mats = mats_in;
+    t.device = ctx.device;
     t.alignment = alignment ? alignment : 1;
     t.H = mats_in.back().h;
     t.depth = log2u(t.H);

@@ -136,11 +136,46 @@ struct Seg {
     const uint64_t *src;
     uint64_t len;
     uint64_t dst;
+    uint64_t padded;  // words len..padded are zero
 };
 __global__ void gather_kernel(const Seg *segs, uint64_t n, uint64_t *out) {
     for (uint64_t s = blockIdx.x; s < n; s += gridDim.x) {
         Seg g = segs[s];
-        for (uint64_t i = threadIdx.x; i < g.len; i += blockDim.x) out[g.dst + i] = g.src[i];
+        for (uint64_t i = threadIdx.x; i < g.padded; i += blockDim.x) out[g.dst + i] = i < g.len ? g.src[i] : 0;
+    }
+}
+// The segments' words, padded, one behind the other, into host memory: one
+// gather and one copy per 2^24 words (openings are hundreds of rows and
+// digests; a copy each took about 10 us). Memory of another device than the
+// context's, which a kernel here may not reach, is copied piece by piece.
+inline void gather_to_host(Ctx &ctx, std::vector<Seg> &segs, uint64_t *host, int device) {
+    constexpr uint64_t kWords = 1ull << 24;
+    if (device != ctx.device) {
+        for (const Seg &g : segs) {
+            ctx.d2h(host, g.src, g.len);
+            for (uint64_t k = g.len; k < g.padded; k++) host[k] = 0;
+            host += g.padded;
+        }
+        ctx.sync();
+        return;
+    }
+    for (size_t i = 0; i < segs.size();) {
+        size_t e = i;
+        uint64_t words = 0;
+        for (; e < segs.size() && (e == i || words + segs[e].padded <= kWords); e++)
+            segs[e].dst = words, words += segs[e].padded;
+        std::vector<uint64_t> raw((e - i) * (sizeof(Seg) / 8));
+        memcpy(raw.data(), &segs[i], (e - i) * sizeof(Seg));
+        DBuf up = ctx.upload(raw), out = ctx.alloc(words);
+        if (words) {
+            gather_kernel<<<(unsigned)std::min<size_t>(e - i, 65535), 128, 0, ctx.stream>>>((const Seg *)up.p, e - i, out.p);
+            CK(cudaGetLastError());
+            ctx.launches++;
+            ctx.d2h(host, out.p, words);
+            ctx.sync();
+        }
+        host += words;
+        i = e;
     }
 }
 
@@ -981,13 +1016,13 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
     std::vector<Seg> segs;
     uint64_t total = 0;
     for (auto &p : plans) {
-        for (auto &r : p.rows) segs.push_back({r.src, r.len, total}), total += r.len;
-        for (auto *s : p.sibs) segs.push_back({s, 4, total}), total += 4;
+        for (auto &r : p.rows) segs.push_back({r.src, r.len, total, r.len}), total += r.len;
+        for (auto *s : p.sibs) segs.push_back({s, 4, total, 4}), total += 4;
     }
     const uint64_t *gathered = nullptr;  // pinned staging (the gathered hints)
     if (!segs.empty()) {
         DBuf d_out = ctx.alloc(total);
-        std::vector<uint64_t> raw(segs.size() * 3);
+        std::vector<uint64_t> raw(segs.size() * (sizeof(Seg) / 8));
         memcpy(raw.data(), segs.data(), segs.size() * sizeof(Seg));
         DBuf up = ctx.upload(raw);
         L(gather_kernel, (unsigned)std::min<size_t>(segs.size(), 65535), 128, 0, (const Seg *)up.p, (uint64_t)segs.size(),

@@ -61,3 +61,16 @@ def test_large_tree_with_another_table_matches_oracle(product, diag):
         del gt
     finally:
         ctx.close()
+
+
+def test_openings_across_gather_chunks(product, gpu_ctx):
+    """prove_batch gathers at most 2^24 words at a time: 2^14 rows of 1025
+    words, padded to 1032, cross that line inside the row list."""
+    rng = np.random.default_rng(3)
+    m = rng.integers(0, P, size=(1 << 14, 1025), dtype=np.uint64)
+    gt = product.LmcsTree(gpu_ctx, [product.to_device(m)], 8)
+    fields, commits = gt.prove_batch(range(1 << 14))
+    want = np.zeros((1 << 14, 1032), dtype=np.uint64)
+    want[:, :1025] = m
+    assert np.array_equal(fields.reshape(1 << 14, 1032), want)
+    assert commits.shape[0] == 0
