@@ -416,7 +416,7 @@ struct LdePlan {
     uint32_t L = 0, log_blowup = 0;
     uint64_t h = 0;
     std::vector<uint32_t> sizes;  // bit ranges, ascending
-    const TwTables *tw = nullptr;
+    const TwTables *tw = nullptr, *coset_tw = nullptr;  // roots of order 2^L and 2^(L + log_blowup)
     uint32_t scale_lo_bits = 0;
     uint64_t scale_hi_len = 0;
     DBuf scale_lo, scale_hi;  // every coset's two-level table of (s*w_{hB}^c)^i / h
@@ -434,6 +434,7 @@ inline LdePlan lde_plan(Ctx &ctx, uint64_t h, uint32_t log_blowup, uint64_t shif
     p.h = h;
     p.log_blowup = log_blowup;
     p.tw = &ctx.twiddles(p.L);
+    p.coset_tw = &ctx.twiddles(p.L + log_blowup);
     auto tuned = ctx.lde_split.find(p.L);
     p.sizes = tuned != ctx.lde_split.end() ? tuned->second : pass_sizes(p.L);
     p.scale_lo_bits = p.L < 12 ? p.L : 12;
@@ -466,40 +467,84 @@ inline LdePlan lde_plan(Ctx &ctx, uint64_t h, uint32_t log_blowup, uint64_t shif
     return p;
 }
 
-// KT: the range's bit count as a template argument (0 = read at run time);
-// the common 8-column ranges of 7..10 bits get their own instances, whose
-// round loops and index arithmetic fold at compile time.
-template <int C, bool DIF, int KT = 0>
+template <int C, bool DIF>
 inline void launch_lde_pass(Ctx &ctx, const lde::PassArgs &a, uint64_t groups, unsigned n_blocks_y) {
     const uint32_t G = 1u << a.k;
     const unsigned threads = (G >= 8 ? G / 8 : 1) * C;
     const size_t smem = ((size_t)G * C + G) * 8;
     static std::atomic<uint64_t> attr_done{0};
-    smem_attr_once(attr_done, lde::lde_pass_kernel<C, DIF, KT>, (1024 * C + 1024) * 8);
-    lde::lde_pass_kernel<C, DIF, KT><<<dim3((unsigned)(groups * a.n_tiles), n_blocks_y), threads, smem, ctx.stream>>>(a);
+    smem_attr_once(attr_done, lde::lde_pass_kernel<C, DIF>, (1024 * C + 1024) * 8);
+    lde::lde_pass_kernel<C, DIF><<<dim3((unsigned)(groups * a.n_tiles), n_blocks_y), threads, smem, ctx.stream>>>(a);
     CK(cudaGetLastError());
     ctx.launches++;
 }
-template <int C, int KT = 0>
+template <int C>
 inline void launch_lde_fused(Ctx &ctx, const lde::FusedArgs &a, uint64_t groups) {
     const uint32_t G = 1u << a.k;
     const unsigned threads = (G >= 8 ? G / 8 : 1) * C;
     const size_t smem = (2 * (size_t)G * C + 3 * (size_t)G) * 8;
     static std::atomic<uint64_t> attr_done{0};
-    smem_attr_once(attr_done, lde::lde_fused_kernel<C, KT>, (2 * 1024 * C + 3 * 1024) * 8);
-    lde::lde_fused_kernel<C, KT><<<(unsigned)(groups * a.n_tiles), threads, smem, ctx.stream>>>(a);
+    smem_attr_once(attr_done, lde::lde_fused_kernel<C>, (2 * 1024 * C + 3 * 1024) * 8);
+    lde::lde_fused_kernel<C><<<(unsigned)(groups * a.n_tiles), threads, smem, ctx.stream>>>(a);
+    CK(cudaGetLastError());
+    ctx.launches++;
+}
+// Tile kernels: blocks per group such that a block takes several tiles (its
+// tables built once) but the launch still has at least about kTileThreads
+// threads, eight rounds of what the chip holds.
+constexpr uint64_t kTileThreads = 148ull * 2048 * 8;
+inline uint32_t tile_step(uint64_t groups, uint32_t n_tiles, uint32_t threads, uint32_t ny) {
+    const uint64_t want = (kTileThreads / threads + groups * ny - 1) / (groups * ny);
+    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(n_tiles, want));
+}
+template <bool DIF, int KT>
+inline void launch_lde_pass_tile(Ctx &ctx, lde::PassArgs a, uint64_t groups, unsigned ny) {
+    constexpr uint32_t G = 1u << KT;
+    constexpr int smem = (G * 8 + G) * 8;
+    static std::atomic<uint64_t> attr_done{0};
+    smem_attr_once(attr_done, lde::lde_pass_tile_kernel<DIF, KT>, smem);
+    a.tile_step = tile_step(groups, a.n_tiles, G, ny);
+    lde::lde_pass_tile_kernel<DIF, KT><<<dim3((unsigned)(groups * a.tile_step), ny), G, smem, ctx.stream>>>(a);
+    CK(cudaGetLastError());
+    ctx.launches++;
+}
+template <int KT>
+inline void launch_lde_fused_tile(Ctx &ctx, lde::FusedArgs a, uint64_t groups) {
+    constexpr uint32_t G = 1u << KT;
+    constexpr int smem = (G * 8 + 4 * G) * 8;
+    static std::atomic<uint64_t> attr_done{0};
+    smem_attr_once(attr_done, lde::lde_fused_tile_kernel<KT>, smem);
+    a.tile_step = tile_step(groups, a.n_tiles, G, 1);
+    lde::lde_fused_tile_kernel<KT><<<(unsigned)(groups * a.tile_step), G, smem, ctx.stream>>>(a);
     CK(cudaGetLastError());
     ctx.launches++;
 }
 template <bool DIF>
 inline void launch_lde_pass_any(Ctx &ctx, uint32_t C, const lde::PassArgs &a, uint64_t groups, unsigned ny) {
-    if (C == 2) launch_lde_pass<2, DIF>(ctx, a, groups, ny);
-    else if (C == 4) launch_lde_pass<4, DIF>(ctx, a, groups, ny);
-    else if (a.k == 7) launch_lde_pass<8, DIF, 7>(ctx, a, groups, ny);
-    else if (a.k == 8) launch_lde_pass<8, DIF, 8>(ctx, a, groups, ny);
-    else if (a.k == 9) launch_lde_pass<8, DIF, 9>(ctx, a, groups, ny);
-    else if (a.k == 10) launch_lde_pass<8, DIF, 10>(ctx, a, groups, ny);
-    else launch_lde_pass<8, DIF>(ctx, a, groups, ny);
+    if (C == 2) return launch_lde_pass<2, DIF>(ctx, a, groups, ny);
+    if (C == 4) return launch_lde_pass<4, DIF>(ctx, a, groups, ny);
+    switch (a.k) {
+        case 5: return launch_lde_pass_tile<DIF, 5>(ctx, a, groups, ny);
+        case 6: return launch_lde_pass_tile<DIF, 6>(ctx, a, groups, ny);
+        case 7: return launch_lde_pass_tile<DIF, 7>(ctx, a, groups, ny);
+        case 8: return launch_lde_pass_tile<DIF, 8>(ctx, a, groups, ny);
+        case 9: return launch_lde_pass_tile<DIF, 9>(ctx, a, groups, ny);
+        case 10: return launch_lde_pass_tile<DIF, 10>(ctx, a, groups, ny);
+        default: return launch_lde_pass<8, DIF>(ctx, a, groups, ny);
+    }
+}
+inline void launch_lde_fused_any(Ctx &ctx, uint32_t C, const lde::FusedArgs &a, uint64_t groups) {
+    if (C == 2) return launch_lde_fused<2>(ctx, a, groups);
+    if (C == 4) return launch_lde_fused<4>(ctx, a, groups);
+    switch (a.k) {
+        case 5: return launch_lde_fused_tile<5>(ctx, a, groups);
+        case 6: return launch_lde_fused_tile<6>(ctx, a, groups);
+        case 7: return launch_lde_fused_tile<7>(ctx, a, groups);
+        case 8: return launch_lde_fused_tile<8>(ctx, a, groups);
+        case 9: return launch_lde_fused_tile<9>(ctx, a, groups);
+        case 10: return launch_lde_fused_tile<10>(ctx, a, groups);
+        default: return launch_lde_fused<8>(ctx, a, groups);
+    }
 }
 
 // in: h x w (row stride ld_in) -> out: (h << log_blowup) x w (row stride
@@ -547,6 +592,7 @@ inline void lde_run(Ctx &ctx, const LdePlan &p, const uint64_t *d_in, uint64_t l
         f.log_cosets = p.log_blowup;
         f.inv_root = inv;
         f.fwd_root = fwd;
+        f.coset_root = ntt::PowTab{p.coset_tw->fwd_lo.p, p.coset_tw->fwd_hi.p, p.coset_tw->lo_bits};
         f.scale_lo = p.scale_lo.p;
         f.scale_hi = p.scale_hi.p;
         f.scale_lo_bits = p.scale_lo_bits;
@@ -555,13 +601,7 @@ inline void lde_run(Ctx &ctx, const LdePlan &p, const uint64_t *d_in, uint64_t l
         f.cp_hi = p.colpow_hi.p;
         f.cp_lo_bits = p.colpow_lo_bits;
         f.cp_hi_len = p.colpow_hi_len;
-        if (C == 2) launch_lde_fused<2>(ctx, f, h >> f.k);
-        else if (C == 4) launch_lde_fused<4>(ctx, f, h >> f.k);
-        else if (f.k == 7) launch_lde_fused<8, 7>(ctx, f, h >> f.k);
-        else if (f.k == 8) launch_lde_fused<8, 8>(ctx, f, h >> f.k);
-        else if (f.k == 9) launch_lde_fused<8, 9>(ctx, f, h >> f.k);
-        else if (f.k == 10) launch_lde_fused<8, 10>(ctx, f, h >> f.k);
-        else launch_lde_fused<8>(ctx, f, h >> f.k);
+        launch_lde_fused_any(ctx, C, f, h >> f.k);
     }
     for (int i = (int)n - 2; i >= 0; i--) {  // forward transform, low ranges, every coset
         lde::PassArgs a{};

@@ -25,6 +25,7 @@ namespace gl {
 
 constexpr uint64_t P = 0xFFFFFFFF00000001ULL;
 constexpr uint64_t EPS = 0xFFFFFFFFULL;  // 2^64 mod p
+constexpr uint64_t R = EPS;              // Montgomery radix 2^64 mod p
 constexpr uint64_t W = 7;                // EF non-residue
 constexpr uint64_t GEN = 7;              // multiplicative generator
 
@@ -159,6 +160,35 @@ __device__ __forceinline__ uint64_t mul_weak(uint64_t a, uint64_t b) {
     mul128_dev(a, b, r0, r1, r2, r3);
     return reduce4_dev(r0, r1, r2, r3);
 }
+#if !defined(__CUDACC_RTC__)
+// (r3 r2 r1 r0) / 2^64 mod p, below 2^64 (below p when the value is below
+// 2^64 p): Montgomery reduction with p^-1 = 1 + 2^32 mod 2^64. With l, h the
+// halves of the value, a = l + (l << 32) mod 2^64 and e the carry of that sum,
+// h - (a - (a >> 32) - e) is the result, plus p when it borrows.
+__device__ __forceinline__ uint64_t mont_reduce_dev(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+    uint32_t o0, o1;
+    asm("{\n\t.reg .u32 a1, b0, b1, m;\n\t"
+        "add.cc.u32 a1, %3, %2;\n\t"
+        "addc.u32 m, a1, 0;\n\t"     // (a >> 32) + e, no wrap
+        "sub.cc.u32 b0, %2, m;\n\t"
+        "subc.u32 b1, a1, 0;\n\t"
+        "sub.cc.u32 %0, %4, b0;\n\t"
+        "subc.cc.u32 %1, %5, b1;\n\t"
+        "subc.u32 m, 0, 0;\n\t"      // borrow: 0xFFFFFFFF = eps
+        "sub.cc.u32 %0, %0, m;\n\t"  // + p = - eps (mod 2^64)
+        "subc.u32 %1, %1, 0;\n\t}"
+        : "=&r"(o0), "=&r"(o1)
+        : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
+    return ((uint64_t)o1 << 32) | o0;
+}
+// (a * b + c) / 2^64 mod p for words below 2^64; canonical when
+// the sum is below 2^64 p. 16 instructions (four 32x32-bit products)
+// without c, against 20 for the plain weak product and 26 for the canonical.
+__device__ __forceinline__ uint64_t mont_mul(uint64_t a, uint64_t b, uint64_t c = 0) {
+    const unsigned __int128 v = (unsigned __int128)a * b + c;
+    return mont_reduce_dev((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)(v >> 64), (uint32_t)(v >> 96));
+}
+#endif
 // Wide value lo + hi * 2^64 (below 2^96), an integer congruent mod p: a chain
 // of sums and differences accumulates here and is reduced once at its end.
 struct Wide {

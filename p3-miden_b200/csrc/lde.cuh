@@ -36,16 +36,32 @@
 // shifts, not multiplications. The powers t^e of every round are built once
 // per block in a shared table (2^k - 1 entries per direction).
 //
-// All values stay canonical (< p).
+// All values stay canonical (< p). Twiddles and scales are kept in Montgomery
+// form (times R = 2^64): a product with one is a Montgomery product, 16
+// instructions and canonical, against 26 for a canonical plain product. As
+// R^3 = 1 mod p, a product of two plain table words comes into that form by
+// one Montgomery product and one bare reduction (mont_of).
 #pragma once
 #include "gl.cuh"
 #include "ntt.cuh"
 
 namespace lde {
 
-__device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) { return gl::add_dev(a, b); }
+// a + b as a - (p - b): seven instructions against nine for add_dev (p - b
+// = p when b = 0; the borrow then adds p back)
+__device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) { return gl::sub_dev(a, gl::P - b); }
 __device__ __forceinline__ uint64_t sub(uint64_t a, uint64_t b) { return gl::sub_dev(a, b); }
-__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) { return gl::mul(a, b); }
+// a times the word whose Montgomery form is m
+__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t m) { return gl::mont_mul(a, m); }
+// Montgomery form of x * y: x y R^-1, then R^-1 once more (R^-2 = R)
+__device__ __forceinline__ uint64_t mont_of(uint64_t x, uint64_t y) {
+    const uint64_t v = gl::mont_mul(x, y);
+    return gl::mont_reduce_dev((uint32_t)v, (uint32_t)(v >> 32), 0, 0);
+}
+// Montgomery form of a table's power
+__device__ __forceinline__ uint64_t mont_at(const ntt::PowTab &t, uint64_t e) {
+    return mont_of(__ldg(t.lo + (e & ((1ull << t.lo_bits) - 1))), __ldg(t.hi + (e >> t.lo_bits)));
+}
 
 // x * 2^S mod p (canonical) for x < 2^64 and S in {24, 48}: the 128-bit
 // product (x >> (64 - S)) * 2^64 + (x << S) reduced with 2^64 = eps and
@@ -225,7 +241,7 @@ __device__ void fill_table(uint64_t *T, uint32_t k, uint32_t blo, uint64_t base_
             const uint32_t li = r == 3 ? rel / 7 : r == 2 ? rel / 3 : rel;
             const uint32_t e = rel - li * em1 + 1;
             const uint64_t l = base_lo + ((uint64_t)li << blo);
-            Tr[rel] = root.at(((l * e) & emask) << (L - b - r));
+            Tr[rel] = mont_at(root, ((l * e) & emask) << (L - b - r));
         }
     }
 }
@@ -263,13 +279,10 @@ __device__ __forceinline__ void round(uint64_t *sm, const uint64_t *T, uint32_t 
 
 // All rounds of a k-bit range; every round ends with a block barrier.
 // tw_low: whether the round at bit 0 has a nontrivial table (base_lo != 0).
-template <int C, bool DIF, int KT = 0>
-__device__ __forceinline__ void run_rounds(uint64_t *sm, const uint64_t *T, bool tw_low, uint32_t k_rt, uint32_t c,
-                                           uint32_t t, uint32_t TPC_rt) {
-    const uint32_t k = KT ? (uint32_t)KT : k_rt;
-    const uint32_t TPC = KT ? (1u << KT) / 8 : TPC_rt;
+template <int C, bool DIF>
+__device__ __forceinline__ void run_rounds(uint64_t *sm, const uint64_t *T, bool tw_low, uint32_t k, uint32_t c,
+                                           uint32_t t, uint32_t TPC) {
     const uint32_t nr = (k + 2) / 3;
-#pragma unroll
     for (uint32_t rd = 0; rd < nr; rd++) {
         uint32_t q_lo, r;
         round_bits(DIF, k, rd, q_lo, r);
@@ -289,6 +302,7 @@ struct PassArgs {
     uint64_t w;                   // columns
     uint32_t L, blo, k;           // transform size 2^L; range [blo, blo + k)
     uint32_t n_tiles;             // column tiles; blockIdx.x = group * n_tiles + tile
+    uint32_t tile_step;           // tile kernels: blocks per group; blockIdx.x = group * tile_step + first tile
     uint32_t src_bitrev;          // position i is read from row bitrev_L(i)
     ntt::PowTab root;             // powers of w_h (forward) or w_h^-1 (inverse)
 };
@@ -298,9 +312,10 @@ struct FusedArgs {
     uint64_t *dst;
     uint64_t ld_src, ld_dst;
     uint64_t w;
-    uint32_t L, blo, k, n_tiles, src_bitrev;
+    uint32_t L, blo, k, n_tiles, tile_step, src_bitrev;
     uint32_t log_cosets;          // B = 2^log_cosets output cosets of h rows each
     ntt::PowTab inv_root, fwd_root;
+    ntt::PowTab coset_root;       // powers of w_{hB} (tile kernel)
     // scale of coset c: coefficient i times scale_lo[c*2^lo_bits + (i mod 2^lo_bits)] *
     // scale_hi[c*scale_hi_len + (i >> lo_bits)] = (s*w_{hB}^c)^i / h
     const uint64_t *scale_lo, *scale_hi;
@@ -319,19 +334,20 @@ __device__ __forceinline__ void group_of(uint64_t g, uint32_t blo, uint32_t k, u
     base_lo = base & (S - 1);
 }
 
-// One range of the inverse (DIF = false) or forward (DIF = true) transform;
-// KT != 0 fixes the range's bit count at compile time (blockDim = 2^KT / 8 * C).
-template <int C, bool DIF, int KT = 0>
+// One range of the inverse (DIF = false) or forward (DIF = true) transform,
+// any bit count: narrow matrices (C < 8) and ranges of fewer than
+// kTileMinBits bits.
+template <int C, bool DIF>
 __global__ void __launch_bounds__(1024) lde_pass_kernel(const __grid_constant__ PassArgs a) {
     extern __shared__ uint64_t sm[];
-    const uint32_t kk = KT ? (uint32_t)KT : a.k;
+    const uint32_t kk = a.k;
     const uint32_t G = 1u << kk;
     uint64_t *T = sm + (size_t)G * C;
     const uint32_t tile = blockIdx.x % a.n_tiles;
     uint64_t base, base_lo;
     group_of(blockIdx.x / a.n_tiles, a.blo, kk, base, base_lo);
     const uint64_t col0 = (uint64_t)tile * C;
-    const uint32_t tid = threadIdx.x, c = tid % C, t = tid / C, TPC = KT ? G / 8 : blockDim.x / C;
+    const uint32_t tid = threadIdx.x, c = tid % C, t = tid / C, TPC = blockDim.x / C;
     const bool col_ok = col0 + c < a.w;
     const uint64_t *src = a.src + blockIdx.y * a.src_blk + col0 + c;
     uint64_t *dst = a.dst + blockIdx.y * a.dst_blk + col0 + c;
@@ -342,7 +358,7 @@ __global__ void __launch_bounds__(1024) lde_pass_kernel(const __grid_constant__ 
     }
     fill_table<DIF>(T, kk, a.blo, base_lo, a.L, a.root, tid, blockDim.x);
     __syncthreads();
-    run_rounds<C, DIF, KT>(sm, T, base_lo != 0, kk, c, t, TPC);
+    run_rounds<C, DIF>(sm, T, base_lo != 0, kk, c, t, TPC);
     if (!col_ok) return;
     for (uint32_t m = t; m < G; m += TPC) {
         const uint64_t P = base + ((uint64_t)m << a.blo);
@@ -352,17 +368,17 @@ __global__ void __launch_bounds__(1024) lde_pass_kernel(const __grid_constant__ 
 
 // The top range: inverse rounds, then per coset the scale and the forward
 // rounds, written to the coset's block of the output.
-template <int C, int KT = 0>
+template <int C>
 __global__ void __launch_bounds__(1024) lde_fused_kernel(const __grid_constant__ FusedArgs a) {
     extern __shared__ uint64_t sm[];
-    const uint32_t kk = KT ? (uint32_t)KT : a.k;
+    const uint32_t kk = a.k;
     const uint32_t G = 1u << kk;
     uint64_t *A = sm, *Bf = A + (size_t)G * C, *Ti = Bf + (size_t)G * C, *Tf = Ti + G, *sc = Tf + G;
     const uint32_t tile = blockIdx.x % a.n_tiles;
     uint64_t base, base_lo;
     group_of(blockIdx.x / a.n_tiles, a.blo, kk, base, base_lo);
     const uint64_t col0 = (uint64_t)tile * C;
-    const uint32_t tid = threadIdx.x, c = tid % C, t = tid / C, TPC = KT ? G / 8 : blockDim.x / C;
+    const uint32_t tid = threadIdx.x, c = tid % C, t = tid / C, TPC = blockDim.x / C;
     const uint64_t col = col0 + c;
     const bool col_ok = col < a.w;
     for (uint32_t m = t; m < G; m += TPC) {
@@ -373,7 +389,7 @@ __global__ void __launch_bounds__(1024) lde_fused_kernel(const __grid_constant__
     fill_table<false>(Ti, kk, a.blo, base_lo, a.L, a.inv_root, tid, blockDim.x);
     fill_table<true>(Tf, kk, a.blo, base_lo, a.L, a.fwd_root, tid, blockDim.x);
     __syncthreads();
-    run_rounds<C, false, KT>(A, Ti, base_lo != 0, kk, c, t, TPC);
+    run_rounds<C, false>(A, Ti, base_lo != 0, kk, c, t, TPC);
     const uint64_t h = 1ull << a.L;
     const uint32_t B = 1u << a.log_cosets;
     const uint64_t lo_mask = (1ull << a.scale_lo_bits) - 1;
@@ -382,21 +398,20 @@ __global__ void __launch_bounds__(1024) lde_fused_kernel(const __grid_constant__
         const uint64_t *shi = a.scale_hi + cs * a.scale_hi_len;
         for (uint32_t m = tid; m < G; m += blockDim.x) {
             const uint64_t P = base + ((uint64_t)m << a.blo);
-            sc[m] = mul(__ldg(slo + (P & lo_mask)), __ldg(shi + (P >> a.scale_lo_bits)));
+            sc[m] = mont_of(__ldg(slo + (P & lo_mask)), __ldg(shi + (P >> a.scale_lo_bits)));
         }
         __syncthreads();
         for (uint32_t m = t; m < G; m += TPC) {
             uint64_t v = mul(A[m * C + c], sc[m]);
             if (a.cp_lo && col_ok) {
                 const uint64_t P = base + ((uint64_t)m << a.blo), tc = col / 2;
-                const uint64_t f = mul(__ldg(a.cp_lo + (tc << a.cp_lo_bits) + (P & ((1ull << a.cp_lo_bits) - 1))),
-                                       __ldg(a.cp_hi + tc * a.cp_hi_len + (P >> a.cp_lo_bits)));
-                v = mul(v, f);
+                v = mul(v, mont_of(__ldg(a.cp_lo + (tc << a.cp_lo_bits) + (P & ((1ull << a.cp_lo_bits) - 1))),
+                                   __ldg(a.cp_hi + tc * a.cp_hi_len + (P >> a.cp_lo_bits))));
             }
             Bf[m * C + c] = v;
         }
         __syncthreads();
-        run_rounds<C, true, KT>(Bf, Tf, base_lo != 0, kk, c, t, TPC);
+        run_rounds<C, true>(Bf, Tf, base_lo != 0, kk, c, t, TPC);
         if (col_ok) {
             uint64_t *dst = a.dst + (uint64_t)gl::bitrev(cs, a.log_cosets) * h * a.ld_dst + col;
             for (uint32_t m = t; m < G; m += TPC) {
@@ -406,6 +421,217 @@ __global__ void __launch_bounds__(1024) lde_fused_kernel(const __grid_constant__
         }
         // the next coset writes sc (not read by the stores) and, after a
         // barrier, Bf
+    }
+}
+
+// ---------------------------------------------------------- tile kernels
+// The same two kernels for 8-column tiles and a bit count fixed at compile
+// time, bound by the integer pipes. A thread keeps its 8 elements of a column
+// in registers from global memory through the first round and from the last
+// round to global memory; only the rounds between go through shared memory
+// (two exchanges for 7..9 bits instead of four), and all index arithmetic is
+// compile-time offsets from a few pointers. A block takes several column
+// tiles of its group, so the twiddle table is built once for them.
+// The fused kernel holds the coefficients in registers: the last inverse
+// round and the first forward round work on the same elements
+// (t + j * 2^(k-3)), and coset c's scale (s w_{hB}^c)^i / h is the previous
+// one's times w_{hB}^i, one product per element and coset from one table.
+// Measured, 2^18 x 336, blowup 2 (B200): see the launcher in context.cuh.
+constexpr int kTileMinBits = 5;
+
+// Element m of column c: rows are paired into 128-byte lines, and the half a
+// row takes is the parity of its low four bits, so that the two rows a
+// half-warp touches in any round lie in different halves.
+__device__ __forceinline__ uint32_t row_parity(uint32_t m) { return __popc(m & 15) & 1; }
+__host__ __device__ constexpr uint32_t cparity(uint32_t m) { return (m ^ (m >> 1) ^ (m >> 2) ^ (m >> 3)) & 1; }
+
+template <int KT, bool DIF, int RD>
+struct Round {
+    static constexpr int NR = (KT + 2) / 3;
+    static constexpr int HI = KT - 3 * RD;
+    static constexpr int Q = DIF ? (HI >= 3 ? HI - 3 : 0) : 3 * RD;
+    static constexpr int R = DIF ? HI - Q : (KT - Q < 3 ? KT - Q : 3);
+    static constexpr int E = 1 << R, N = 8 >> R;  // elements of a task, tasks of a thread
+    static constexpr uint32_t TPC = 1u << (KT - 3);
+    // first element of task i of thread t
+    static __device__ __forceinline__ uint32_t first(uint32_t t, int i) {
+        const uint32_t task = t + i * TPC, low = task & ((1u << Q) - 1);
+        return low | ((task >> Q) << (Q + R));
+    }
+    // v[i * E + e] = element first(t, i) + e * 2^Q
+    template <bool LOAD>
+    static __device__ __forceinline__ void exchange(uint64_t *sm, uint64_t *v, uint32_t t, uint32_t c) {
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const uint32_t m = first(t, i), par = row_parity(m);
+            uint64_t *line = sm + (m >> 1) * 16 + c, *h0 = line + par * 8, *h1 = line + 8 - par * 8;
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                uint64_t *p = (cparity((e << Q) & 15) ? h1 : h0) + ((e << Q) >> 1) * 16;
+                if (LOAD) v[i * E + e] = *p;
+                else *p = v[i * E + e];
+            }
+        }
+    }
+    // T: the range's table; tw_low: whether the round at bit 0 has twiddles
+    static __device__ __forceinline__ void run(uint64_t *v, const uint64_t *T, bool tw_low, uint32_t t) {
+        const uint64_t *Tr = T + ((1u << Q) - 1);
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            uint64_t *x = v + i * E;
+            const uint64_t *Tl = Tr + ((t + i * TPC) & ((1u << Q) - 1)) * (E - 1);
+            if (!DIF && (Q != 0 || tw_low)) {
+#pragma unroll
+                for (int p = 1; p < E; p++) x[p] = mul(x[p], Tl[brev(p, R) - 1]);
+            }
+            if (DIF) dft_dif<R>(x);
+            else dft_dit<R>(x);
+            if (DIF && (Q != 0 || tw_low)) {
+#pragma unroll
+                for (int p = 1; p < E; p++) x[p] = mul(x[p], Tl[brev(p, R) - 1]);
+            }
+        }
+    }
+};
+// Rounds RD.. of a range: on entry v holds the inputs of round RD in its
+// order, on return the outputs of the last round in that one's order.
+template <int KT, bool DIF, int RD = 0>
+__device__ __forceinline__ void tile_rounds(uint64_t *sm, const uint64_t *T, bool tw_low, uint64_t *v, uint32_t t,
+                                            uint32_t c) {
+    using Rd = Round<KT, DIF, RD>;
+    Rd::run(v, T, tw_low, t);
+    if constexpr (RD + 1 < Rd::NR) {
+        Rd::template exchange<false>(sm, v, t, c);
+        __syncthreads();
+        Round<KT, DIF, RD + 1>::template exchange<true>(sm, v, t, c);
+        tile_rounds<KT, DIF, RD + 1>(sm, T, tw_low, v, t, c);
+    }
+}
+
+template <bool DIF, int KT>
+__global__ void __launch_bounds__(1 << KT) lde_pass_tile_kernel(const __grid_constant__ PassArgs a) {
+    extern __shared__ uint64_t sm[];
+    constexpr uint32_t G = 1u << KT;
+    uint64_t *T = sm + (size_t)G * 8;
+    using First = Round<KT, DIF, 0>;
+    using Last = Round<KT, DIF, First::NR - 1>;
+    const uint32_t group = blockIdx.x / a.tile_step;
+    uint64_t base, base_lo;
+    group_of(group, a.blo, KT, base, base_lo);
+    const uint32_t c = threadIdx.x % 8, t = threadIdx.x / 8;
+    fill_table<DIF>(T, KT, a.blo, base_lo, a.L, a.root, threadIdx.x, G);
+    const uint64_t *src = a.src + blockIdx.y * a.src_blk + c;
+    uint64_t *dst = a.dst + blockIdx.y * a.dst_blk + c;
+    for (uint32_t tile = blockIdx.x % a.tile_step; tile < a.n_tiles; tile += a.tile_step) {
+        const uint64_t col0 = (uint64_t)tile * 8;
+        const bool col_ok = col0 + c < a.w;
+        uint64_t v[8];
+#pragma unroll
+        for (int i = 0; i < First::N; i++) {
+            // rows of the task, ascending; read in bit-reversed order, bit b
+            // of e in the position is bit L - 1 - blo - Q - b of the row
+            const uint64_t pos = base + ((uint64_t)First::first(t, i) << a.blo);
+            const uint64_t *p = src + (a.src_bitrev ? gl::bitrev(pos, a.L) : pos) * a.ld_src + col0;
+            const uint64_t step = a.ld_src << (a.src_bitrev ? a.L - a.blo - First::Q - First::R : a.blo + First::Q);
+            uint64_t x[First::E];
+#pragma unroll
+            for (int e = 0; e < First::E; e++) x[e] = col_ok ? __ldg(p + e * step) : 0;
+#pragma unroll
+            for (int e = 0; e < First::E; e++) v[i * First::E + e] = a.src_bitrev ? x[brev(e, First::R)] : x[e];
+        }
+        __syncthreads();  // the table; the last tile's reads
+        tile_rounds<KT, DIF>(sm, T, base_lo != 0, v, t, c);
+        if (col_ok) {
+#pragma unroll
+            for (int i = 0; i < Last::N; i++) {
+                uint64_t *p = dst + (base + ((uint64_t)Last::first(t, i) << a.blo)) * a.ld_dst + col0;
+                const uint64_t step = a.ld_dst << (a.blo + Last::Q);
+#pragma unroll
+                for (int e = 0; e < Last::E; e++) p[e * step] = v[i * Last::E + e];
+            }
+        }
+    }
+}
+
+template <int KT>
+__global__ void __launch_bounds__(1 << KT) lde_fused_tile_kernel(const __grid_constant__ FusedArgs a) {
+    extern __shared__ uint64_t sm[];
+    constexpr uint32_t G = 1u << KT, TPC = G / 8;
+    uint64_t *Ti = sm + (size_t)G * 8, *Tf = Ti + G, *s0 = Tf + G, *om = s0 + G;
+    using First = Round<KT, false, 0>;
+    using LastI = Round<KT, false, First::NR - 1>;
+    using LastF = Round<KT, true, First::NR - 1>;
+    const uint32_t group = blockIdx.x / a.tile_step;
+    uint64_t base, base_lo;
+    group_of(group, a.blo, KT, base, base_lo);
+    const uint32_t c = threadIdx.x % 8, t = threadIdx.x / 8;
+    fill_table<false>(Ti, KT, a.blo, base_lo, a.L, a.inv_root, threadIdx.x, G);
+    fill_table<true>(Tf, KT, a.blo, base_lo, a.L, a.fwd_root, threadIdx.x, G);
+    const uint64_t h = 1ull << a.L;
+    const uint32_t B = 1u << a.log_cosets;
+    {
+        // coset 0's scale s^i / h and the step to the next coset's, w_{hB}^i
+        const uint32_t m = threadIdx.x;
+        const uint64_t pos = base + ((uint64_t)m << a.blo), lo = pos & ((1ull << a.scale_lo_bits) - 1),
+                       hi = pos >> a.scale_lo_bits;
+        s0[m] = mont_of(__ldg(a.scale_lo + lo), __ldg(a.scale_hi + hi));
+        om[m] = mont_at(a.coset_root, pos);
+    }
+    for (uint32_t tile = blockIdx.x % a.tile_step; tile < a.n_tiles; tile += a.tile_step) {
+        const uint64_t col = (uint64_t)tile * 8 + c;
+        const bool col_ok = col < a.w;
+        uint64_t v[8], x[8];
+#pragma unroll
+        for (int i = 0; i < First::N; i++) {
+            const uint64_t pos = base + ((uint64_t)First::first(t, i) << a.blo);
+            const uint64_t *p = a.src + (a.src_bitrev ? gl::bitrev(pos, a.L) : pos) * a.ld_src + col;
+            const uint64_t step = a.ld_src << (a.src_bitrev ? a.L - a.blo - First::Q - First::R : a.blo + First::Q);
+#pragma unroll
+            for (int e = 0; e < First::E; e++) x[i * First::E + e] = col_ok ? __ldg(p + e * step) : 0;
+#pragma unroll
+            for (int e = 0; e < First::E; e++)
+                v[i * First::E + e] = a.src_bitrev ? x[i * First::E + brev(e, First::R)] : x[i * First::E + e];
+        }
+        __syncthreads();  // the tables; the last tile's reads
+        tile_rounds<KT, false>(sm, Ti, base_lo != 0, v, t, c);
+        // v[i * E + e] is element t + (i + e * N) * TPC
+#pragma unroll
+        for (int i = 0; i < LastI::N; i++)
+#pragma unroll
+            for (int e = 0; e < LastI::E; e++) x[i + e * LastI::N] = v[i * LastI::E + e];
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[j] = mul(x[j], s0[t + j * TPC]);
+        if (a.cp_lo && col_ok) {
+            const uint64_t tc = col / 2;
+            const uint64_t *clo = a.cp_lo + (tc << a.cp_lo_bits), *chi = a.cp_hi + tc * a.cp_hi_len;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const uint64_t pos = base + ((uint64_t)(t + j * TPC) << a.blo);
+                x[j] = mul(x[j], mont_of(__ldg(clo + (pos & ((1ull << a.cp_lo_bits) - 1))),
+                                         __ldg(chi + (pos >> a.cp_lo_bits))));
+            }
+        }
+#pragma unroll 1
+        for (uint32_t cs = 0; cs < B; cs++) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = x[j];
+            __syncthreads();  // the last round's reads
+            tile_rounds<KT, true>(sm, Tf, base_lo != 0, v, t, c);
+            if (col_ok) {
+                uint64_t *dst = a.dst + (uint64_t)gl::bitrev(cs, a.log_cosets) * h * a.ld_dst + col;
+#pragma unroll
+                for (int i = 0; i < LastF::N; i++) {
+                    uint64_t *p = dst + (base + ((uint64_t)LastF::first(t, i) << a.blo)) * a.ld_dst;
+                    const uint64_t step = a.ld_dst << (a.blo + LastF::Q);
+#pragma unroll
+                    for (int e = 0; e < LastF::E; e++) p[e * step] = v[i * LastF::E + e];
+                }
+            }
+            if (cs + 1 < B) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) x[j] = mul(x[j], om[t + j * TPC]);
+            }
+        }
     }
 }
 

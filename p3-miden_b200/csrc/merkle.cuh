@@ -37,32 +37,8 @@ struct W {  // lo + hi * 2^64
     uint64_t lo;
     uint32_t hi;
 };
-// (r3 r2 r1 r0) / 2^64 mod p, below 2^64 (below p when the value is below
-// 2^64 p): Montgomery reduction with p^-1 = 1 + 2^32 mod 2^64. With l, h the
-// halves of the value, a = l + (l << 32) mod 2^64 and e the carry of that sum,
-// h - (a - (a >> 32) - e) is the result, plus p when it borrows.
-__device__ __forceinline__ uint64_t mont_reduce(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-    uint32_t o0, o1;
-    asm("{\n\t.reg .u32 a1, b0, b1, m;\n\t"
-        "add.cc.u32 a1, %3, %2;\n\t"
-        "addc.u32 m, a1, 0;\n\t"     // (a >> 32) + e, no wrap
-        "sub.cc.u32 b0, %2, m;\n\t"
-        "subc.u32 b1, a1, 0;\n\t"
-        "sub.cc.u32 %0, %4, b0;\n\t"
-        "subc.cc.u32 %1, %5, b1;\n\t"
-        "subc.u32 m, 0, 0;\n\t"      // borrow: 0xFFFFFFFF = eps
-        "sub.cc.u32 %0, %0, m;\n\t"  // + p = - eps (mod 2^64)
-        "subc.u32 %1, %1, 0;\n\t}"
-        : "=&r"(o0), "=&r"(o1)
-        : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
-    return ((uint64_t)o1 << 32) | o0;
-}
-// a * b / 2^64 mod p. 16 instructions (four 32x32-bit products) against 20
-// for the product with the plain reduction (gl::mul_weak).
-__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) {
-    const unsigned __int128 v = (unsigned __int128)a * b;
-    return mont_reduce((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)(v >> 64), (uint32_t)(v >> 96));
-}
+// a * b / 2^64 mod p, weakly reduced
+__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) { return gl::mont_mul(a, b); }
 __device__ __forceinline__ uint64_t canon(uint64_t a) { return gl::canon_dev(a); }
 // weak + canonical: one wrap at most (a + c - 2^64 + eps < 2^64)
 __device__ __forceinline__ uint64_t add_c(uint64_t a, uint64_t c) {
@@ -141,11 +117,6 @@ __device__ __forceinline__ uint64_t mul_add_w(uint64_t a, uint64_t b, W c) {
         : "r"((uint32_t)a), "r"((uint32_t)(a >> 32)), "r"((uint32_t)b), "r"((uint32_t)(b >> 32)),
           "r"((uint32_t)c.lo), "r"((uint32_t)(c.lo >> 32)), "r"(c.hi));
     return gl::reduce4_dev(r0, r1, r2, r3);
-}
-// (a * b + c) / 2^64 mod p for a 64-bit c (c = C * 2^64 mod p adds C)
-__device__ __forceinline__ uint64_t mul_add_m(uint64_t a, uint64_t b, uint64_t c) {
-    const unsigned __int128 v = (unsigned __int128)a * b + c;
-    return mont_reduce((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)(v >> 64), (uint32_t)(v >> 96));
 }
 // M4 = circ(2,3,1,1) on sums modulo 2^64 and on 32-bit sums
 template <typename T>
@@ -235,7 +206,7 @@ __device__ __forceinline__ void p2_permute_dev(uint64_t *s) {
             const uint64_t c = gl::sub_dev(gl::reduce4_dev(0, 0, (uint32_t)acc.lo, (uint32_t)(acc.lo >> 32)),
                                            (uint64_t)acc.hi << 32);
 #pragma unroll
-            for (int i = 0; i < 12; i++) s[i] = p2w::mul_add_m(s[i], c_p2[p2::OFF_DIAG_M + i], c);
+            for (int i = 0; i < 12; i++) s[i] = gl::mont_mul(s[i], c_p2[p2::OFF_DIAG_M + i], c);
         }
     }
 }

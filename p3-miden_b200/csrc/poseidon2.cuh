@@ -20,10 +20,9 @@ constexpr int OFF_INIT = 0, OFF_TERM = 48, OFF_INT = 96, OFF_DIAG = 118;
 // products that are reduced as a * b / R.
 constexpr int OFF_DIAG_M = N_PARAMS, OFF_MU0P1_M = OFF_DIAG_M + 12, N_DEVICE = OFF_MU0P1_M + 1;
 inline void device_table(const uint64_t *params, uint64_t *out) {
-    constexpr uint64_t R = 0xFFFFFFFFull;  // 2^64 mod p
     for (int i = 0; i < N_PARAMS; i++) out[i] = params[i];
-    for (int i = 0; i < 12; i++) out[OFF_DIAG_M + i] = gl::mul(params[OFF_DIAG + i] % gl::P, R);
-    out[OFF_MU0P1_M] = gl::add(out[OFF_DIAG_M], R);
+    for (int i = 0; i < 12; i++) out[OFF_DIAG_M + i] = gl::mul(params[OFF_DIAG + i] % gl::P, gl::R);
+    out[OFF_MU0P1_M] = gl::add(out[OFF_DIAG_M], gl::R);
 }
 
 // Host permutation with lazy reduction: words stay below 2^64 (congruent
