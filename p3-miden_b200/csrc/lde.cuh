@@ -63,54 +63,17 @@ __device__ __forceinline__ uint64_t mont_at(const ntt::PowTab &t, uint64_t e) {
     return mont_of(__ldg(t.lo + (e & ((1ull << t.lo_bits) - 1))), __ldg(t.hi + (e >> t.lo_bits)));
 }
 
-// x * 2^S mod p (canonical) for x < 2^64 and S in {24, 48}: the 128-bit
-// product (x >> (64 - S)) * 2^64 + (x << S) reduced with 2^64 = eps and
-// 2^96 = -1 on carry chains; the last step folds the carry and the
-// comparison with p into one select.
-template <int S>
-__device__ __forceinline__ uint64_t shl(uint64_t x) {
-    static_assert(S == 24 || S == 48, "shift");
+// x * 2^24 mod p (canonical): (x >> 40) * 2^64 + (x << 24) reduced with
+// 2^64 = eps; the last step folds the carry and the comparison with p into
+// one select.
+__device__ __forceinline__ uint64_t mul_2_24(uint64_t x) {
     const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32);
-    uint32_t l0, l1, h0, h1;  // x << S = (l1:l0), x >> (64 - S) = (h1:h0)
-    if (S == 24) {
-        l0 = x0 << 24;
-        l1 = __funnelshift_l(x0, x1, 24);
-        h0 = x1 >> 8;
-        h1 = 0;
-    } else {
-        l0 = 0;
-        l1 = x0 << 16;
-        h0 = __funnelshift_r(x0, x1, 16);
-        h1 = x1 >> 16;
-    }
     uint32_t r0, r1;
-    if (S == 24) {  // h1 = 0: the generic form's first five instructions do nothing
-        asm("{\n\t.reg .u32 m, u0, u1, t0, t1;\n\t.reg .pred q;\n\t"
-            "sub.cc.u32 u0, 0, %4;\n\t"    // h0*eps
-            "subc.u32 u1, %4, 0;\n\t"
-            "add.cc.u32 %0, %2, u0;\n\t"
-            "addc.cc.u32 %1, %3, u1;\n\t"
-            "addc.u32 m, 0, 0;\n\t"
-            "add.cc.u32 t0, %0, 0xFFFFFFFF;\n\t"  // r + eps: r - p, or the value of a wrapped sum
-            "addc.cc.u32 t1, %1, 0;\n\t"
-            "addc.u32 m, m, 0;\n\t"
-            "setp.ne.u32 q, m, 0;\n\t"
-            "selp.b32 %0, t0, %0, q;\n\t"
-            "selp.b32 %1, t1, %1, q;\n\t}"
-            : "=&r"(r0), "=&r"(r1)
-            : "r"(l0), "r"(l1), "r"(h0));
-        return ((uint64_t)r1 << 32) | r0;
-    }
     asm("{\n\t.reg .u32 m, u0, u1, t0, t1;\n\t.reg .pred q;\n\t"
-        "sub.cc.u32 %0, %2, %5;\n\t"   // (l1:l0) - h1
-        "subc.cc.u32 %1, %3, 0;\n\t"
-        "subc.u32 m, 0, 0;\n\t"
-        "sub.cc.u32 %0, %0, m;\n\t"    // on borrow subtract eps
-        "subc.u32 %1, %1, 0;\n\t"
-        "sub.cc.u32 u0, 0, %4;\n\t"    // + h0*eps
+        "sub.cc.u32 u0, 0, %4;\n\t"    // h0*eps
         "subc.u32 u1, %4, 0;\n\t"
-        "add.cc.u32 %0, %0, u0;\n\t"
-        "addc.cc.u32 %1, %1, u1;\n\t"
+        "add.cc.u32 %0, %2, u0;\n\t"
+        "addc.cc.u32 %1, %3, u1;\n\t"
         "addc.u32 m, 0, 0;\n\t"
         "add.cc.u32 t0, %0, 0xFFFFFFFF;\n\t"  // r + eps: r - p, or the value of a wrapped sum
         "addc.cc.u32 t1, %1, 0;\n\t"
@@ -119,29 +82,46 @@ __device__ __forceinline__ uint64_t shl(uint64_t x) {
         "selp.b32 %0, t0, %0, q;\n\t"
         "selp.b32 %1, t1, %1, q;\n\t}"
         : "=&r"(r0), "=&r"(r1)
-        : "r"(l0), "r"(l1), "r"(h0), "r"(h1));
+        : "r"(x0 << 24), "r"(__funnelshift_l(x0, x1, 24)), "r"(x1 >> 8));
     return ((uint64_t)r1 << 32) | r0;
 }
-
-// x * 2^72 mod p (canonical) for x < 2^64. With (a1:a0) = (x << 8) mod 2^64
-// and y = x >> 56, x * 2^72 = (x << 8) * 2^64 = (a0 - y) * 2^32 - (a0 + a1)
-// mod p (2^64 = eps, 2^128 = -2^32). That value lies in (-2^41, p), so the
-// borrow of one subtraction decides the only correction (+p). Ten
-// instructions in place of shl<48>(shl<24>(x)).
-__device__ __forceinline__ uint64_t shl72(uint64_t x) {
-    const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32);
-    const uint32_t a0 = x0 << 8, a1 = __funnelshift_l(x0, x1, 8), y = x1 >> 24;
+// Divisions by 2^s, s < 64, for x < p: x - m p with m = x p^-1 mod 2^s is a
+// multiple of 2^s, and (x - m p) / 2^s lies in (-p, p), so one conditional
+// addition of p makes it canonical. p^-1 = 1 + 2^32 (mod 2^64).
+//
+// x * 2^-24 = -x * 2^72: m = x mod 2^24 = l, (x >> 24) + l 2^8 - l 2^40.
+__device__ __forceinline__ uint64_t div_2_24(uint64_t x) {
+    const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32), s = x0 << 8;  // l << 8
     uint32_t r0, r1;
-    asm("{\n\t.reg .u32 s0, s1, m;\n\t"
-        "add.cc.u32 s0, %2, %3;\n\t"   // s = a0 + a1 + y * 2^32
-        "addc.u32 s1, %4, 0;\n\t"
-        "sub.cc.u32 %0, 0, s0;\n\t"    // (a0 : 0) - s, borrow when negative
-        "subc.cc.u32 %1, %2, s1;\n\t"
-        "subc.u32 m, 0, 0;\n\t"        // borrow: m = 0xFFFFFFFF = eps
-        "sub.cc.u32 %0, %0, m;\n\t"    // negative: + p = - eps (mod 2^64)
+    asm("{\n\t.reg .u32 m;\n\t"
+        "add.cc.u32 %0, %2, %4;\n\t"
+        "addc.u32 %1, %3, 0;\n\t"
+        "sub.cc.u32 %1, %1, %4;\n\t"
+        "subc.u32 m, 0, 0;\n\t"      // borrow: 0xFFFFFFFF = eps
+        "sub.cc.u32 %0, %0, m;\n\t"  // + p = - eps (mod 2^64)
         "subc.u32 %1, %1, 0;\n\t}"
         : "=&r"(r0), "=&r"(r1)
-        : "r"(a0), "r"(a1), "r"(y));
+        : "r"(__funnelshift_r(x0, x1, 24)), "r"(x1 >> 24), "r"(s));
+    return ((uint64_t)r1 << 32) | r0;
+}
+// x * 2^-48 = -x * 2^48: with t = x0 + x1 (33 bits), m = (t mod 2^16) 2^32 + x0
+// and the quotient is (t >> 16) + (t mod 2^16) 2^16 - m 2^16; the first two
+// terms are t's low word rotated by 16 plus its carry times 2^16. 13
+// instructions against 19 for x * 2^48 from its 112-bit product.
+__device__ __forceinline__ uint64_t div_2_48(uint64_t x) {
+    const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32);
+    uint32_t t, c, r0, r1;
+    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=&r"(t), "=&r"(c) : "r"(x0), "r"(x1));
+    asm("{\n\t.reg .u32 m;\n\t"
+        "add.cc.u32 %0, %2, %3;\n\t"
+        "addc.u32 %1, 0, 0;\n\t"
+        "sub.cc.u32 %0, %0, %4;\n\t"
+        "subc.cc.u32 %1, %1, %5;\n\t"
+        "subc.u32 m, 0, 0;\n\t"
+        "sub.cc.u32 %0, %0, m;\n\t"
+        "subc.u32 %1, %1, 0;\n\t}"
+        : "=&r"(r0), "=&r"(r1)
+        : "r"(__funnelshift_l(t, t, 16)), "r"(c << 16), "r"(x0 << 16), "r"(__byte_perm(x0, t, 0x5432)));
     return ((uint64_t)r1 << 32) | r0;
 }
 
@@ -156,20 +136,20 @@ template <int R>
 __device__ __forceinline__ void dft_dif(uint64_t *x) {
     if (R == 3) {
         const uint64_t a0 = add(x[0], x[4]), a4 = sub(x[0], x[4]);
-        const uint64_t a1 = add(x[1], x[5]), a5 = shl<24>(sub(x[5], x[1]));          // * w8 = -2^24
-        const uint64_t a2 = add(x[2], x[6]), a6 = shl<48>(sub(x[2], x[6]));          // * w8^2 = 2^48
-        const uint64_t a3 = add(x[3], x[7]), a7 = shl72(sub(x[7], x[3]));  // * w8^3 = -2^72
+        const uint64_t a1 = add(x[1], x[5]), a5 = mul_2_24(sub(x[5], x[1]));  // * w8 = -2^24
+        const uint64_t a2 = add(x[2], x[6]), a6 = div_2_48(sub(x[6], x[2]));  // * w8^2 = 2^48
+        const uint64_t a3 = add(x[3], x[7]), a7 = div_2_24(sub(x[3], x[7]));  // * w8^3 = -2^72
         const uint64_t b0 = add(a0, a2), b2 = sub(a0, a2);
-        const uint64_t b1 = add(a1, a3), b3 = shl<48>(sub(a1, a3));
+        const uint64_t b1 = add(a1, a3), b3 = div_2_48(sub(a3, a1));
         const uint64_t b4 = add(a4, a6), b6 = sub(a4, a6);
-        const uint64_t b5 = add(a5, a7), b7 = shl<48>(sub(a5, a7));
+        const uint64_t b5 = add(a5, a7), b7 = div_2_48(sub(a7, a5));
         x[0] = add(b0, b1), x[1] = sub(b0, b1);
         x[2] = add(b2, b3), x[3] = sub(b2, b3);
         x[4] = add(b4, b5), x[5] = sub(b4, b5);
         x[6] = add(b6, b7), x[7] = sub(b6, b7);
     } else if (R == 2) {
         const uint64_t a0 = add(x[0], x[2]), a2 = sub(x[0], x[2]);
-        const uint64_t a1 = add(x[1], x[3]), a3 = shl<48>(sub(x[1], x[3]));  // * w4 = 2^48
+        const uint64_t a1 = add(x[1], x[3]), a3 = div_2_48(sub(x[3], x[1]));  // * w4 = 2^48
         x[0] = add(a0, a1), x[1] = sub(a0, a1);
         x[2] = add(a2, a3), x[3] = sub(a2, a3);
     } else {
@@ -184,25 +164,25 @@ __device__ __forceinline__ void dft_dit(uint64_t *x) {
         const uint64_t a2 = add(x[2], x[3]), a3 = sub(x[2], x[3]);
         const uint64_t a4 = add(x[4], x[5]), a5 = sub(x[4], x[5]);
         const uint64_t a6 = add(x[6], x[7]), a7 = sub(x[6], x[7]);
-        uint64_t v = shl<48>(a3);  // * w4^-1 = -2^48
+        uint64_t v = div_2_48(a3);  // * w4^-1 = -2^48
         const uint64_t c0 = add(a0, a2), c2 = sub(a0, a2);
-        const uint64_t c1 = sub(a1, v), c3 = add(a1, v);
-        v = shl<48>(a7);
+        const uint64_t c1 = add(a1, v), c3 = sub(a1, v);
+        v = div_2_48(a7);
         const uint64_t c4 = add(a4, a6), c6 = sub(a4, a6);
-        const uint64_t c5 = sub(a5, v), c7 = add(a5, v);
+        const uint64_t c5 = add(a5, v), c7 = sub(a5, v);
         x[0] = add(c0, c4), x[4] = sub(c0, c4);
-        v = shl72(c5);  // * w8^-1 = 2^72
-        x[1] = add(c1, v), x[5] = sub(c1, v);
-        v = shl<48>(c6);  // * w8^-2 = -2^48
-        x[2] = sub(c2, v), x[6] = add(c2, v);
-        v = shl<24>(c7);  // * w8^-3 = 2^24
+        v = div_2_24(c5);  // * w8^-1 = 2^72, negated
+        x[1] = sub(c1, v), x[5] = add(c1, v);
+        v = div_2_48(c6);  // * w8^-2 = -2^48
+        x[2] = add(c2, v), x[6] = sub(c2, v);
+        v = mul_2_24(c7);  // * w8^-3 = 2^24
         x[3] = add(c3, v), x[7] = sub(c3, v);
     } else if (R == 2) {
         const uint64_t a0 = add(x[0], x[1]), a1 = sub(x[0], x[1]);
         const uint64_t a2 = add(x[2], x[3]), a3 = sub(x[2], x[3]);
-        const uint64_t v = shl<48>(a3);  // * w4^-1 = -2^48
+        const uint64_t v = div_2_48(a3);  // * w4^-1 = -2^48
         x[0] = add(a0, a2), x[2] = sub(a0, a2);
-        x[1] = sub(a1, v), x[3] = add(a1, v);
+        x[1] = add(a1, v), x[3] = sub(a1, v);
     } else {
         const uint64_t a0 = add(x[0], x[1]), a1 = sub(x[0], x[1]);
         x[0] = a0, x[1] = a1;
