@@ -416,7 +416,8 @@ __global__ void __launch_bounds__(1024) lde_fused_kernel(const __grid_constant__
 // round and the first forward round work on the same elements
 // (t + j * 2^(k-3)), and coset c's scale (s w_{hB}^c)^i / h is the previous
 // one's times w_{hB}^i, one product per element and coset from one table.
-// Measured, 2^18 x 336, blowup 2 (B200): see the launcher in context.cuh.
+// Measured (B200): 2^18 x 336, blowup 2, 5.55 -> 3.53 ms; 2^20 x 37, blowup
+// 8, 9.57 -> 6.0 ms, with the ALU pipe at 76..79 % of its peak.
 constexpr int kTileMinBits = 5;
 
 // Element m of column c: rows are paired into 128-byte lines, and the half a
@@ -488,8 +489,11 @@ __device__ __forceinline__ void tile_rounds(uint64_t *sm, const uint64_t *T, boo
     }
 }
 
+// 1536 resident threads per SM (at most 40 registers; 1024 threads with 62
+// registers measured 4 % slower on 2^18 x 2633); the fused kernel, with the
+// coefficients in registers, keeps 1024.
 template <bool DIF, int KT>
-__global__ void __launch_bounds__(1 << KT) lde_pass_tile_kernel(const __grid_constant__ PassArgs a) {
+__global__ void __launch_bounds__(1 << KT, 1536 >> KT) lde_pass_tile_kernel(const __grid_constant__ PassArgs a) {
     extern __shared__ uint64_t sm[];
     constexpr uint32_t G = 1u << KT;
     uint64_t *T = sm + (size_t)G * 8;
@@ -534,7 +538,7 @@ __global__ void __launch_bounds__(1 << KT) lde_pass_tile_kernel(const __grid_con
 }
 
 template <int KT>
-__global__ void __launch_bounds__(1 << KT) lde_fused_tile_kernel(const __grid_constant__ FusedArgs a) {
+__global__ void __launch_bounds__(1 << KT, 1024 >> KT) lde_fused_tile_kernel(const __grid_constant__ FusedArgs a) {
     extern __shared__ uint64_t sm[];
     constexpr uint32_t G = 1u << KT, TPC = G / 8;
     uint64_t *Ti = sm + (size_t)G * 8, *Tf = Ti + G, *s0 = Tf + G, *om = s0 + G;
