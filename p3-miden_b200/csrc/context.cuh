@@ -370,18 +370,6 @@ inline void transpose(Ctx &ctx, const uint64_t *in, uint64_t ld, uint64_t *out, 
     ctx.launches++;
 }
 
-// Host-built two-level power table of v for exponents < 2^L.
-inline void pow_table(uint64_t v, uint32_t L, uint32_t lo_bits, std::vector<uint64_t> &out_lo,
-                      std::vector<uint64_t> &out_hi) {
-    size_t nlo = 1ull << lo_bits, nhi = 1ull << (L > lo_bits ? L - lo_bits : 0);
-    out_lo.resize(nlo);
-    out_hi.resize(nhi);
-    uint64_t x = 1;
-    for (size_t i = 0; i < nlo; i++) out_lo[i] = x, x = gl::mul(x, v);
-    uint64_t y = 1;
-    for (size_t i = 0; i < nhi; i++) out_hi[i] = y, y = gl::mul(y, x);
-}
-
 // A split of L bits into LDE bit ranges is valid when every range has 1..10
 // bits (the kernels' shared-memory groups) and the ranges add up to L.
 inline bool valid_split(uint32_t L, const std::vector<uint32_t> &sizes) {
@@ -408,10 +396,39 @@ inline std::vector<uint32_t> pass_sizes(uint32_t L) {
     return v;
 }
 
+// Two-level power tables of an LDE plan. Row y < n_scale: coset y's scale
+// (shift * step^y)^i / h; row n_scale + t: powers of col_base[t]. A row is
+// its low table (exponents below 2^lo_bits) followed by its high table
+// (multiples of 2^lo_bits); one thread per entry, one power each.
+struct PlanTables {
+    static constexpr uint32_t kMaxCols = 8;
+    uint32_t n_scale, n_cols, scale_lo_bits, col_lo_bits;
+    uint64_t scale_hi_len, col_hi_len;
+    uint64_t shift, step, h_inv;
+    uint64_t col_base[kMaxCols];
+    uint64_t *scale_lo, *scale_hi, *col_lo, *col_hi;
+};
+__global__ void __launch_bounds__(128) plan_tables_kernel(const __grid_constant__ PlanTables a) {
+    const uint32_t y = blockIdx.y;
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool scale = y < a.n_scale;
+    const uint32_t row = scale ? y : y - a.n_scale, lo_bits = scale ? a.scale_lo_bits : a.col_lo_bits;
+    const uint64_t n_lo = 1ull << lo_bits, n_hi = scale ? a.scale_hi_len : a.col_hi_len;
+    if (e >= n_lo + n_hi) return;
+    const uint64_t base = scale ? gl::mul(a.shift, gl::pow(a.step, row)) : a.col_base[row];
+    if (e < n_lo) {
+        const uint64_t v = gl::pow(base, e);
+        (scale ? a.scale_lo : a.col_lo)[row * n_lo + e] = scale ? gl::mul(v, a.h_inv) : v;
+    } else {
+        (scale ? a.scale_hi : a.col_hi)[row * n_hi + (e - n_lo)] = gl::pow(base, (e - n_lo) << lo_bits);
+    }
+}
+
 // Bit-reversed coset LDE of an h x w matrix, split into a plan (tables on
-// the device; synchronises the context stream once) and launches (no host
-// synchronisation, any stream), so that column slabs of one trace can be
-// transformed while earlier slabs are hashed.
+// the device, filled on the context stream) and launches (no host
+// synchronisation, any stream that has waited for the context stream), so
+// that column slabs of one trace can be transformed while earlier slabs are
+// hashed.
 struct LdePlan {
     uint32_t L = 0, log_blowup = 0;
     uint64_t h = 0;
@@ -437,33 +454,41 @@ inline LdePlan lde_plan(Ctx &ctx, uint64_t h, uint32_t log_blowup, uint64_t shif
     p.coset_tw = &ctx.twiddles(p.L + log_blowup);
     auto tuned = ctx.lde_split.find(p.L);
     p.sizes = tuned != ctx.lde_split.end() ? tuned->second : pass_sizes(p.L);
+    // the scale and column tables are made on the device, by one kernel on
+    // the context stream (host-made ones took 0.1 to 0.4 ms and three
+    // synchronisations per call)
+    const uint32_t B = 1u << log_blowup;
     p.scale_lo_bits = p.L < 12 ? p.L : 12;
-    const uint64_t wb = gl::root(p.L + log_blowup);
-    const uint64_t hinv = gl::inv(h % gl::P);
-    std::vector<uint64_t> lo, hi, all_lo, all_hi;
-    uint64_t sk = shift;
-    for (uint64_t k = 0; k < (1ull << log_blowup); k++) {
-        pow_table(sk, p.L, p.scale_lo_bits, lo, hi);
-        for (auto &v : lo) v = gl::mul(v, hinv);  // the inverse transform's 1/h
-        all_lo.insert(all_lo.end(), lo.begin(), lo.end());
-        all_hi.insert(all_hi.end(), hi.begin(), hi.end());
-        p.scale_hi_len = hi.size();
-        sk = gl::mul(sk, wb);
-    }
-    p.scale_lo = ctx.upload(all_lo);
-    p.scale_hi = ctx.upload(all_hi);
+    p.scale_hi_len = 1ull << (p.L - p.scale_lo_bits);
+    p.scale_lo = ctx.alloc((size_t)B << p.scale_lo_bits);
+    p.scale_hi = ctx.alloc((size_t)B * p.scale_hi_len);
+    PlanTables a{};
+    a.n_scale = B;
+    a.scale_lo_bits = p.scale_lo_bits;
+    a.scale_hi_len = p.scale_hi_len;
+    a.shift = shift;
+    a.step = gl::root(p.L + log_blowup);
+    a.h_inv = gl::inv(h % gl::P);
+    a.scale_lo = p.scale_lo.p;
+    a.scale_hi = p.scale_hi.p;
     if (!col_bases.empty()) {
+        if (col_bases.size() > PlanTables::kMaxCols) throw CudaError{ERR_INVALID, "too many column bases"};
         p.colpow_lo_bits = p.L < 10 ? p.L : 10;
         p.colpow_hi_len = 1ull << (p.L - p.colpow_lo_bits);
-        all_lo.clear(), all_hi.clear();
-        for (uint64_t cb : col_bases) {
-            pow_table(cb, p.L, p.colpow_lo_bits, lo, hi);
-            all_lo.insert(all_lo.end(), lo.begin(), lo.end());
-            all_hi.insert(all_hi.end(), hi.begin(), hi.end());
-        }
-        p.colpow_lo = ctx.upload(all_lo);
-        p.colpow_hi = ctx.upload(all_hi);
+        p.colpow_lo = ctx.alloc(col_bases.size() << p.colpow_lo_bits);
+        p.colpow_hi = ctx.alloc(col_bases.size() * p.colpow_hi_len);
+        a.n_cols = (uint32_t)col_bases.size();
+        a.col_lo_bits = p.colpow_lo_bits;
+        a.col_hi_len = p.colpow_hi_len;
+        for (size_t i = 0; i < col_bases.size(); i++) a.col_base[i] = col_bases[i];
+        a.col_lo = p.colpow_lo.p;
+        a.col_hi = p.colpow_hi.p;
     }
+    const uint64_t per = std::max<uint64_t>((1ull << a.scale_lo_bits) + a.scale_hi_len,
+                                            a.n_cols ? (1ull << a.col_lo_bits) + a.col_hi_len : 0);
+    plan_tables_kernel<<<dim3((unsigned)((per + 127) / 128), a.n_scale + a.n_cols), 128, 0, ctx.stream>>>(a);
+    CK(cudaGetLastError());
+    ctx.launches++;
     return p;
 }
 

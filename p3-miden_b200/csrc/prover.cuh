@@ -258,7 +258,15 @@ inline void commit_main_pipelined(Ctx &ctx, const Instance *inst, size_t n_inst,
     std::vector<LdePlan> plans;
     for (size_t i = 0; i < n_inst; i++)
         plans.push_back(lde_plan(ctx, inst[i].height, lb, gl::exp2k(gl::GEN, log_max_h - log2u(inst[i].height))));
-    // allocations and tables are complete once the context stream drained (lde_plan syncs it)
+    // the other streams start behind the allocations and tables of the context stream
+    {
+        cudaEvent_t ready;
+        CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+        CK(cudaEventRecord(ready, ctx.stream));
+        CK(cudaStreamWaitEvent(ctx.lde_stream, ready, 0));
+        CK(cudaStreamWaitEvent(ctx.copy_stream, ready, 0));
+        cudaEventDestroy(ready);
+    }
     std::vector<cudaEvent_t> ev_copy(slabs.size()), ev_lde(slabs.size()), ev_t0(slabs.size());
     for (size_t s = 0; s < slabs.size(); s++) {
         CK(cudaEventCreateWithFlags(&ev_copy[s], cudaEventDisableTiming));
