@@ -697,16 +697,22 @@ inline void launch_tc(Ctx &ctx, std::atomic<uint64_t> &attr_done, K kernel, uint
     ctx.launches++;
 }
 
-// Leaf sponge of one height class of n leaves: one 16-lane group per leaf
-// when the class is small (latency-bound), the tensor-core permutation when
-// it is large, one thread per leaf between.
-constexpr uint64_t kTcLeaves = 1ull << 15;
+// Leaf sponge of one height class of n leaves, by how many lanes fill the
+// chip: 16 per leaf up to 2^11 leaves (latency-bound), four for 2^12 and 2^13,
+// one for 2^14, and the tensor-core permutation from 2^15 on (the figures
+// are at leaf_class_quad_kernel; 2^15 leaves x 512 columns with four lanes
+// each take 2.9 ms against 2.4, 2^16 5.2 against 3.3).
+constexpr uint64_t kTcLeaves = 1ull << 15, kQuadLeaves = 1ull << 13;
 inline void launch_leaf_class(Ctx &ctx, const merkle::ClassArgs &a, uint64_t n) {
     const unsigned coop_blocks = (unsigned)((n * 16 + 127) / 128), blocks = (unsigned)((n + 127) / 128);
     if (a.cm && a.n_mats != 1) throw CudaError{ERR_INVALID, "column-major copy of a multi-matrix class"};
     if (n <= merkle::kCoopLeaves) {
         if (a.cm) merkle::leaf_class_coop_kernel<true><<<coop_blocks, 128, 0, ctx.stream>>>(a);
         else merkle::leaf_class_coop_kernel<false><<<coop_blocks, 128, 0, ctx.stream>>>(a);
+    } else if (n <= kQuadLeaves) {
+        const unsigned quad_blocks = (unsigned)((n * 4 + 127) / 128);
+        if (a.cm) merkle::leaf_class_quad_kernel<true><<<quad_blocks, 128, 0, ctx.stream>>>(a);
+        else merkle::leaf_class_quad_kernel<false><<<quad_blocks, 128, 0, ctx.stream>>>(a);
     } else if (n >= kTcLeaves && ctx.hash_table.p) {
         uint64_t perms = 0;
         for (int m = 0; m < a.n_mats; m++) perms += (a.width[m] + 7) / 8;
@@ -723,12 +729,14 @@ inline void launch_leaf_class(Ctx &ctx, const merkle::ClassArgs &a, uint64_t n) 
 }
 
 // Compress layer 0 (already filled) up to the root (kernels only; the root
-// stays on the device); finish_tree also fetches the root. Levels with at
-// least kWideParents parents run one thread per parent, up to four levels
-// per launch (a block keeps at least a warp's worth of parents per level);
-// levels above 128 parents run one 16-lane group per parent, one launch per
-// level; the last levels (at most 128 parents) run in one cluster launch.
-constexpr uint64_t kWideParents = 8192, kTcParents = 1ull << 16;
+// stays on the device); finish_tree also fetches the root. Levels of at least
+// 2^16 parents run the tensor-core permutation; levels of at least 2^14 one
+// thread per parent, up to four levels per launch (a block keeps at least a
+// warp's worth of parents per level); 2^13 and 2^12 four lanes per parent;
+// levels above 128 parents one 16-lane group per parent, one launch per level
+// (the lanes by the same figures as the leaf classes); the last levels (at
+// most 128 parents) run in one cluster launch.
+constexpr uint64_t kWideParents = 1ull << 14, kTcParents = 1ull << 16, kQuadParents = 1ull << 12;
 inline void compress_layers(Ctx &ctx, Tree &t) {
     uint32_t l = 0;
     for (; ctx.hash_table.p && l < t.depth && (t.H >> (l + 1)) >= kTcParents; l++) {
@@ -746,7 +754,9 @@ inline void compress_layers(Ctx &ctx, Tree &t) {
     }
     while (l < t.depth && (t.H >> (l + 1)) > 128) {
         const uint64_t n_parents = t.H >> (l + 1);
-        merkle::compress_level_coop_kernel<<<(unsigned)((n_parents * 16 + 127) / 128), 128, 0, ctx.stream>>>(
+        if (n_parents >= kQuadParents)
+            merkle::compress_level_quad_kernel<<<(unsigned)(n_parents * 4 / 128), 128, 0, ctx.stream>>>(t.layers.p, t.H, l);
+        else merkle::compress_level_coop_kernel<<<(unsigned)((n_parents * 16 + 127) / 128), 128, 0, ctx.stream>>>(
             t.layers.p, t.H, l);
         CK(cudaGetLastError());
         ctx.launches++;

@@ -293,6 +293,86 @@ __device__ __forceinline__ uint64_t permute(uint64_t x, int l, const uint64_t *s
 }
 }  // namespace p2x
 
+// Permutation shared by 4 lanes, for launches of a few thousand states: lane
+// l holds words l, l + 4 and l + 8 (position l of the three M4 blocks), so an
+// S-box layer is three S-boxes per lane, the block sums are local and M4 is
+// one exchange of the four positions, y_l = 2 v_l + 3 v_{l+1} + v_{l+2} +
+// v_{l+3}. Internal rounds as p2x::permute. About 800 warp instructions per
+// state against 545 for one thread per state and 2450 for 16 lanes; alone, a
+// chained permutation takes 22.0 k cycles against 44.9 and 17.0. 8 states per
+// warp; all 32 lanes must call it. `sc`: p2x::stage_consts.
+namespace p2q {
+__device__ __forceinline__ uint32_t from(uint32_t v, int d) {  // lane l + d of the quad
+    return __shfl_sync(0xffffffffu, v, (threadIdx.x & 3) + d & 3, 4);
+}
+// next: index of the lane's first constant of the next round in sc, or -1
+__device__ __forceinline__ void ext_linear(uint64_t *x, const uint64_t *sc, int next) {
+    const uint32_t h0 = (uint32_t)(x[0] >> 37), h1 = (uint32_t)(x[1] >> 37), h2 = (uint32_t)(x[2] >> 37);
+    const uint64_t tw = x[0] + x[1] + x[2];
+    const uint32_t ts = h0 + h1 + h2;
+    const uint32_t hs[3] = {h0, h1, h2};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const uint64_t v = x[k] + tw;  // the M4 input of block k, sums as in p2w::ext_linear
+        const uint32_t h = hs[k] + ts;
+        uint64_t w = v + v;
+        uint32_t u = h + h;
+#pragma unroll
+        for (int d = 1; d < 4; d++) {
+            const uint64_t vd = ((uint64_t)from((uint32_t)(v >> 32), d) << 32) | from((uint32_t)v, d);
+            const uint32_t hd = from(h, d);
+            w += d == 1 ? vd + vd + vd : vd;
+            u += d == 1 ? 3 * hd : hd;
+        }
+        if (next >= 0) {
+            const uint64_t rc = sc[next + 4 * k];
+            w += rc;
+            u += (uint32_t)(rc >> 37);
+        }
+        x[k] = p2w::fold_wraps(w, u);
+    }
+}
+struct Lane {
+    uint64_t mu[3];   // diagonal words of the lane (0 for word 0)
+    uint64_t mu0p1;   // mu_0 + 1 mod p
+};
+__device__ __forceinline__ Lane lane_consts(const uint64_t *sc, int l) {
+    return Lane{{l ? sc[p2::OFF_DIAG + l] : 0, sc[p2::OFF_DIAG + l + 4], sc[p2::OFF_DIAG + l + 8]},
+                gl::add_dev(sc[p2::OFF_DIAG], 1)};
+}
+__device__ __forceinline__ void permute(uint64_t *x, const uint64_t *sc, const Lane &k) {
+    using namespace p2w;
+    const int l = threadIdx.x & 3;
+    ext_linear(x, sc, p2::OFF_INIT + l);
+#pragma unroll 1
+    for (int r = 0; r < 8; r++) {
+        if (r == 4) {
+            uint64_t z = ((uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(x[0] >> 32), 0, 4) << 32) |
+                         __shfl_sync(0xffffffffu, (uint32_t)x[0], 0, 4);
+            if (l == 0) x[0] = 0;
+#pragma unroll 1
+            for (int q = 0; q < 22; q++) {
+                const uint64_t zs = sbox(add_c(z, sc[p2::OFF_INT + q]));
+                W P = wadd1(wadd1(wide(x[0]), x[1]), x[2]);
+#pragma unroll
+                for (int m = 1; m < 4; m <<= 1) P = wadd(P, p2x::shflW_xor(P, m));
+                z = mul_add_w(zs, k.mu0p1, P);  // P < 11 * 2^64
+                const W t = wadd1(P, zs);       // < 12 * 2^64
+                x[0] = l ? mul_add_w(x[0], k.mu[0], t) : 0;
+                x[1] = mul_add_w(x[1], k.mu[1], t);
+                x[2] = mul_add_w(x[2], k.mu[2], t);
+            }
+            if (l == 0) x[0] = z;
+#pragma unroll
+            for (int i = 0; i < 3; i++) x[i] = add_c(x[i], sc[p2::OFF_TERM + l + 4 * i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) x[i] = sbox(x[i]);
+        ext_linear(x, sc, r < 3 ? p2::OFF_INIT + 12 * (r + 1) + l : r == 3 || r == 7 ? -1 : p2::OFF_TERM + 12 * (r - 3) + l);
+    }
+}
+}  // namespace p2q
+
 namespace merkle {
 
 constexpr int MAX_MATS = 8;
@@ -374,7 +454,7 @@ __global__ void __launch_bounds__(128, 8) leaf_class_kernel(const __grid_constan
 // each of a row's chained permutations costs the full single-thread latency.
 // States are weakly reduced like leaf_class_kernel's (congruent mod p, not
 // always the same words), so classes may mix the two kernels.
-constexpr uint64_t kCoopLeaves = 4096;
+constexpr uint64_t kCoopLeaves = 2048;
 template <bool CM>
 __global__ void __launch_bounds__(128) leaf_class_coop_kernel(const __grid_constant__ ClassArgs a) {
     __shared__ uint64_t sc[p2::N_PARAMS];
@@ -390,10 +470,12 @@ __global__ void __launch_bounds__(128) leaf_class_coop_kernel(const __grid_const
     for (int m = 0; m < a.n_mats; m++) {
         const uint64_t w = a.width[m];
         const uint64_t *row = a.data[m] + (ok ? j : 0) * a.ld[m];
+        uint64_t next = l < 8 && ok && l < w ? __ldg(row + l) : 0;  // loaded a permutation ahead
 #pragma unroll 1
         for (uint64_t i = 0; i < w; i += 8) {
-            if (l < 8) x = ok && i + l < w ? __ldg(row + i + l) : 0;
+            if (l < 8) x = next;
             if (CM && l < 8 && ok && i + l < w && j < a.cm_rows) a.cm[(i + l) * a.cm_ld + j] = x;
+            next = l < 8 && ok && i + 8 + l < w ? __ldg(row + i + 8 + l) : 0;
             x = p2x::permute(x, l, sc, k);
         }
     }
@@ -402,6 +484,53 @@ __global__ void __launch_bounds__(128) leaf_class_coop_kernel(const __grid_const
         if (l < 4) a.digests_out[j * 4 + l] = p2w::canon(x);
     } else if (l < 12) {
         a.states_out[j * 12 + l] = x;
+    }
+}
+
+// The leaf sponge with four lanes per leaf (p2q), for classes of 2^12 and
+// 2^13 leaves: one thread per leaf leaves most schedulers without a warp
+// there, and 16 lanes per leaf more than fill them. Trees of 2^11 / 2^12 /
+// 2^13 / 2^14 leaves x 512 columns took 0.88 / 1.25 / 1.96 / 3.51 ms with 16
+// lanes, 0.93 / 0.94 / 1.15 / 1.85 with four and - / - / 1.68 / 1.72 with one
+// thread. The next chunk's words are loaded before the permutation of this
+// one.
+template <bool CM>
+__global__ void __launch_bounds__(128) leaf_class_quad_kernel(const __grid_constant__ ClassArgs a) {
+    __shared__ uint64_t sc[p2::N_PARAMS];
+    p2x::stage_consts(sc);
+    const int l = threadIdx.x & 3;
+    const p2q::Lane k = p2q::lane_consts(sc, l);
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (((t & ~31ull) >> 2) >> a.log_h) return;  // warp-uniform: the warp's first leaf is past the class
+    const uint64_t j = t >> 2;
+    const bool ok = (j >> a.log_h) == 0;
+    uint64_t x[3] = {0, 0, 0};
+    if (ok && a.prev) {
+        const uint64_t *p = a.prev + (j >> (a.log_h - a.prev_log_h)) * 12 + l;
+        x[0] = p[0], x[1] = p[4], x[2] = p[8];
+    }
+    for (int m = 0; m < a.n_mats; m++) {
+        const uint64_t w = ok ? a.width[m] : 0, n = a.width[m];
+        const uint64_t *row = a.data[m] + (ok ? j : 0) * a.ld[m];
+        uint64_t c0 = l < w ? __ldg(row + l) : 0, c1 = 4 + l < w ? __ldg(row + 4 + l) : 0;
+#pragma unroll 1
+        for (uint64_t i = 0; i < n; i += 8) {
+            x[0] = c0, x[1] = c1;
+            if (CM && j < a.cm_rows) {
+                if (i + l < w) a.cm[(i + l) * a.cm_ld + j] = c0;
+                if (i + 4 + l < w) a.cm[(i + 4 + l) * a.cm_ld + j] = c1;
+            }
+            c0 = i + 8 + l < w ? __ldg(row + i + 8 + l) : 0;
+            c1 = i + 12 + l < w ? __ldg(row + i + 12 + l) : 0;
+            p2q::permute(x, sc, k);
+        }
+    }
+    if (!ok) return;
+    if (a.digests_out) {
+        a.digests_out[j * 4 + l] = p2w::canon(x[0]);
+    } else {
+        uint64_t *p = a.states_out + j * 12 + l;
+        p[0] = x[0], p[4] = x[1], p[8] = x[2];
     }
 }
 
@@ -478,6 +607,19 @@ __global__ void __launch_bounds__(128) compress_level_coop_kernel(uint64_t *laye
     const uint64_t p = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
     const uint64_t n = H >> (l_in + 1);
     compress_parent_coop(layers, 2 * H - 2 * (H >> l_in), 2 * H - 2 * (H >> (l_in + 1)), p, p < n, l, sc, k);
+}
+
+// The same with four lanes per parent (a multiple of 32 parents).
+__global__ void __launch_bounds__(128) compress_level_quad_kernel(uint64_t *layers, uint64_t H, uint32_t l_in) {
+    __shared__ uint64_t sc[p2::N_PARAMS];
+    p2x::stage_consts(sc);
+    const int l = threadIdx.x & 3;
+    const p2q::Lane k = p2q::lane_consts(sc, l);
+    const uint64_t p = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const uint64_t *in = layers + 4 * (2 * H - 2 * (H >> l_in) + 2 * p);
+    uint64_t x[3] = {in[l], in[4 + l], 0};
+    p2q::permute(x, sc, k);
+    layers[4 * (2 * H - 2 * (H >> (l_in + 1)) + p) + l] = p2w::canon(x[0]);
 }
 
 __device__ __forceinline__ void cluster_sync() {

@@ -1,6 +1,7 @@
-"""Trees large enough for the tensor-core permutation (csrc/p2tc.cuh), bit
-for bit against the CPU oracle: block and round edges of its launches, rows
-that end inside a chunk, several matrices and classes, extreme words and a
+"""Trees of the sizes where the hash kernels change (16, 4 and 1 lanes per
+state, csrc/merkle.cuh; the tensor-core permutation, csrc/p2tc.cuh), bit for
+bit against the CPU oracle: block and round edges of the launches, rows that
+end inside a chunk, several matrices and classes, extreme words and a
 non-default permutation table."""
 import numpy as np
 import pytest
@@ -22,6 +23,11 @@ def words(rng, h, w, kind):
 
 
 CASES = [
+    ([(1 << 11, 9)], 8, "edges"),                        # the last class and level of 16 lanes per state
+    ([(1 << 12, 17)], 8, "edges"),                       # four lanes per leaf
+    ([(1 << 9, 4), (1 << 12, 8), (1 << 13, 13), (1 << 13, 1)], 8, "random"),  # carried states, two matrices
+    ([(1 << 13, 3)], 1, "top"),
+    ([(1 << 14, 12)], 8, "edges"),                       # one thread per leaf
     ([(1 << 15, 1)], 1, "random"),                       # two groups per SM, one short chunk
     ([(1 << 15, 8)], 8, "top"),
     ([(1 << 15, 9)], 8, "edges"),                        # a chunk and one word
