@@ -469,10 +469,10 @@ P3G_API int p3g_deep_quotient(p3g_ctx *x, const uint64_t *const *d_mats, const u
         const uint32_t log_lde = p3g::log2u(heights[n_mats - 1]);
         p3g::Launcher L{x->c};
         p3g::DeepOpen st;
-        // the point quotients and weights of the opening, then the assembly
-        (void)p3g::deep_evals(x->c, L, all, log_blowup, log_lde, zs, alignment, st, nullptr);
-        std::vector<uint64_t> ev(evals, evals + 4 * total_w);
-        p3g::DBuf layer = p3g::deep_assemble(x->c, L, all, log_lde, ev, gl::ef{alpha2[0], alpha2[1]},
+        p3g::deep_points(x->c, L, all, log_lde, zs, alignment, st);
+        st.evals = x->c.alloc(4 * total_w);
+        x->c.h2d(st.evals.p, evals, 4 * total_w);
+        p3g::DBuf layer = p3g::deep_assemble(x->c, L, all, log_lde, gl::ef{alpha2[0], alpha2[1]},
                                              gl::ef{beta2[0], beta2[1]}, st);
         CK(cudaMemcpyAsync(d_out, layer.p, (2ull << log_lde) * 8, cudaMemcpyDeviceToDevice, x->c.stream));
         x->c.sync();

@@ -292,10 +292,22 @@ GL_HD uint64_t pow(uint64_t b, uint64_t e) {
     }
     return r;
 }
-GL_HD uint64_t inv(uint64_t a) { return pow(a, P - 2); }
 GL_HD uint64_t exp2k(uint64_t a, unsigned k) {
     while (k--) a = mul(a, a);
     return a;
+}
+// a^(p-2), p - 2 = (2^31 - 1) 2^33 + (2^32 - 1): 73 products (127 by squaring
+// and multiplying along the exponent's 63 ones). 0 gives 0.
+GL_HD uint64_t inv(uint64_t a) {
+    const uint64_t t2 = mul(mul(a, a), a);            // a^(2^2 - 1)
+    const uint64_t t3 = mul(mul(t2, t2), a);
+    const uint64_t t6 = mul(exp2k(t3, 3), t3);
+    const uint64_t t12 = mul(exp2k(t6, 6), t6);
+    const uint64_t t24 = mul(exp2k(t12, 12), t12);
+    const uint64_t t30 = mul(exp2k(t24, 6), t6);
+    const uint64_t t31 = mul(mul(t30, t30), a);
+    const uint64_t t32 = mul(mul(t31, t31), a);
+    return mul(exp2k(t31, 33), t32);
 }
 // primitive 2^k-th root of unity, 7^((p-1)/2^k)
 GL_HD uint64_t root(unsigned k) { return pow(GEN, (P - 1) >> k); }
