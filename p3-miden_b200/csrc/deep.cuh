@@ -32,7 +32,7 @@ struct PQArgs {
 // in the base field, so the batch inversion runs on base-field words: per
 // point and z one square, three products of the batch and two for the
 // quotient, against 12 for products of extension elements. One inversion per
-// 16 quotients (46 -> 21 us at 2^18 points with both changes, B200).
+// 16 quotients (46 -> 20 us at 2^18 points with gl::inv's chain, B200).
 __global__ void __launch_bounds__(128) point_quotients_kernel(const __grid_constant__ PQArgs a) {
     const uint64_t i0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * CHUNK;
     if (i0 >= a.n) return;
@@ -167,8 +167,8 @@ __global__ void __launch_bounds__(512) colsum_finish_kernel(const uint64_t *part
 // The column coefficients -ac^{W-1-c} over the aligned columns of all
 // matrices, and the reduced openings f_red(z_j) = sum_c ac^{W-1-c} f_c(z_j)
 // (padding columns are zero). One block: ac^0..ac^1023 by doubling in shared
-// memory, then 1024 columns at a time from the last (33 us with a power per
-// column, 8 us this way, at 1338 columns).
+// memory, then 1024 columns at a time from the last (at 1338 columns 22 us cold,
+// 33 with a power per column; on the host it was an upload and two waits).
 constexpr int MAX_DOTS = 24;
 struct CoefArgs {
     int n_mats;
@@ -225,8 +225,9 @@ __global__ void __launch_bounds__(1024) coef_kernel(const __grid_constant__ Coef
 
 // Row dot products dots[i] = sum_col coef[col] * M[i][col] (EF coef), G lanes
 // per row (about eight columns per lane at least, so that the reduction over
-// the lanes does not count: 64 columns with 32 lanes per row ran at a third of
-// the rate), coefficients staged in shared memory.
+// the lanes does not count: 2^18 x 64 took 111 us with 32 lanes per row, 47
+// with 8; 2^16 x 250 74 us with 32, 42 with 16), coefficients staged in shared
+// memory. Bound by the integer pipes (two lazy products per word).
 template <int G>
 __global__ void __launch_bounds__(256) rowdot_lanes_kernel(const uint64_t *M, uint64_t h, uint64_t w,
                                                            const uint64_t *coef, uint64_t *dots) {

@@ -122,20 +122,57 @@ __global__ void __launch_bounds__(128) leaf_thread_kernel(const LeafJob *jobs, u
 }
 constexpr uint32_t kThreadLeaves = 2048;  // from this many leaves on, one thread per leaf
 
-// One warp per compression of one tree level.
+// The compressions of one tree level of every proof: 16 lanes each (p2x), or
+// four (p2q), or one thread, by how many there are (launch_compress).
+__device__ __forceinline__ uint64_t child_word(const CJob &job, const uint64_t *pool, int l) {
+    return l < 4 ? pool[4 * (uint64_t)job.left + l] : pool[4 * (uint64_t)job.right + l - 4];
+}
 __global__ void __launch_bounds__(128) compress_kernel(const CJob *jobs, uint32_t n, uint64_t *pool) {
     __shared__ uint64_t sc[p2::N_PARAMS];
     p2x::stage_consts(sc);
     const int l = threadIdx.x & 15;
     const p2x::Lane k = p2x::lane_consts(sc, l);
-    const uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (j >= n) return;  // warp-uniform
-    const CJob job = jobs[j];
-    uint64_t x = 0;
-    if (l < 4) x = pool[4 * (uint64_t)job.left + l];
-    else if (l < 8) x = pool[4 * (uint64_t)job.right + l - 4];
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, j = t >> 4;
+    if ((t & ~31u) >> 4 >= n) return;  // warp-uniform: the warp's first job is past the end
+    const CJob job = jobs[j < n ? j : n - 1];
+    uint64_t x = l < 8 ? child_word(job, pool, l) : 0;
     x = p2x::permute(x, l, sc, k);
-    if (threadIdx.x % 32 < 4) pool[4 * (uint64_t)job.out + l] = p2w::canon(x);
+    if (j < n && l < 4) pool[4 * (uint64_t)job.out + l] = p2w::canon(x);
+}
+__global__ void __launch_bounds__(128) compress_quad_kernel(const CJob *jobs, uint32_t n, uint64_t *pool) {
+    __shared__ uint64_t sc[p2::N_PARAMS];
+    p2x::stage_consts(sc);
+    const int l = threadIdx.x & 3;
+    const p2q::Lane k = p2q::lane_consts(sc, l);
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, j = t >> 2;
+    if ((t & ~31u) >> 2 >= n) return;  // warp-uniform
+    const CJob job = jobs[j < n ? j : n - 1];
+    uint64_t x[3] = {child_word(job, pool, l), child_word(job, pool, l + 4), 0};
+    p2q::permute(x, sc, k);
+    if (j < n) pool[4 * (uint64_t)job.out + l] = p2w::canon(x[0]);
+}
+__global__ void __launch_bounds__(128) compress_thread_kernel(const CJob *jobs, uint32_t n, uint64_t *pool) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    const CJob job = jobs[j];
+    uint64_t s[12];
+#pragma unroll
+    for (int i = 0; i < 12; i++) s[i] = i < 8 ? child_word(job, pool, i) : 0;
+    p2_permute_dev(s);
+#pragma unroll
+    for (int i = 0; i < 4; i++) pool[4 * (uint64_t)job.out + i] = p2w::canon(s[i]);
+}
+// Lanes per compression by the sizes at which they fill the chip, as for the
+// leaf classes (merkle.cuh). A batch of 24 proofs has 30 k compressions on a
+// level: a whole warp each took 0.19 ms a level, a thread each 0.03.
+constexpr uint32_t kCoopJobs = 2048, kQuadJobs = 8192;
+inline void launch_compress(Ctx &ctx, const CJob *jobs, uint32_t n, uint64_t *pool) {
+    if (!n) return;
+    if (n <= kCoopJobs) compress_kernel<<<(n * 16 + 127) / 128, 128, 0, ctx.stream>>>(jobs, n, pool);
+    else if (n <= kQuadJobs) compress_quad_kernel<<<(n * 4 + 127) / 128, 128, 0, ctx.stream>>>(jobs, n, pool);
+    else compress_thread_kernel<<<(n + 127) / 128, 128, 0, ctx.stream>>>(jobs, n, pool);
+    CK(cudaGetLastError());
+    ctx.launches++;
 }
 
 struct DeepArgs {
@@ -149,8 +186,10 @@ struct DeepArgs {
     int32_t *flags;            // flags[0]: a denominator vanished
 };
 // One warp per query: red_row = sum_i v_i * alpha_c^(T-1-i), then
-// de = sum_p bp^p (red_open_p - red_row) / (z_p - x_q).
-__global__ void __launch_bounds__(128) deep_kernel(const __grid_constant__ DeepArgs a) {
+// de = sum_p bp^p (red_open_p - red_row) / (z_p - x_q). Proof blockIdx.y (all
+// proofs of a pass in one launch; one after another they took 20 us each).
+__global__ void __launch_bounds__(128) deep_kernel(const DeepArgs *args) {
+    const DeepArgs &a = args[blockIdx.y];
     const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (q >= a.nq) return;
@@ -209,8 +248,10 @@ struct FriArgs {
     uint32_t final_deg;
     int32_t *flags;            // flags[1]: final polynomial; flags[2 + r]: round r positions
 };
-// One block: rounds in order, entries and rows over the threads.
-__global__ void __launch_bounds__(256) fri_kernel(const __grid_constant__ FriArgs a) {
+// One block per proof (45 us each, now side by side): rounds in order,
+// entries and rows over the threads.
+__global__ void __launch_bounds__(256) fri_kernel(const FriArgs *args) {
+    const FriArgs &a = args[blockIdx.x];
     const uint32_t A = 1u << a.log_a;
     uint64_t *cur = a.cur, *nxt = a.nxt;
     for (uint32_t i = threadIdx.x; i < (a.n_rounds ? a.rounds[0].ncur : a.n_final); i += blockDim.x)
@@ -692,7 +733,7 @@ inline void prepare(const uint64_t *p2, const PcsParams &pcs, const Instance *in
 
 // The device pass over several prepared proofs: one staged upload, the leaf
 // sponges of every proof in one launch, every tree level of every proof in
-// one launch per level, then per proof the DEEP and FRI kernels, and one
+// one launch per level, the DEEP and FRI checks in one launch each, and one
 // read-back of all roots and flags. Proofs decided early are skipped.
 inline void device_pass(Ctx &ctx, const std::vector<Prepared *> &vs, Timing *tm, unsigned threads = 1) {
     struct Seg {
@@ -769,6 +810,10 @@ inline void device_pass(Ctx &ctx, const std::vector<Prepared *> &vs, Timing *tm,
         o_fx[j] = seg(v.final_x.data(), v.final_x.size() * 8);
         o_fp[j] = seg(v.final_poly.data(), v.final_poly.size() * 8);
     }
+    // the DEEP and FRI kernels' arguments, filled once the device buffer is known
+    std::vector<DeepArgs> das;
+    std::vector<FriArgs> fas;
+    const size_t o_das = seg(nullptr, nj * sizeof(DeepArgs)), o_fas = seg(nullptr, nj * sizeof(FriArgs));
     const size_t staged = words;
     const size_t o_hints = seg(hints.data(), hints.size() * 8);  // copied into the pool
     const size_t pool_words = 4 * n_nodes + hints.size() + 4;
@@ -800,32 +845,7 @@ inline void device_pass(Ctx &ctx, const std::vector<Prepared *> &vs, Timing *tm,
         copy();
         for (auto &t : th) t.join();
     }
-    CK(cudaEventRecord(e0, ctx.stream));
-    ctx.h2d(d.p, st, staged);
-    ctx.h2d(pool + 4 * n_nodes, st + o_hints, hints.size());
-    CK(cudaMemsetAsync(back, 0, back_words * 8, ctx.stream));
     int32_t *d_flags = (int32_t *)(back + 4 * n_roots);
-    if (!leaves.empty()) {
-        const uint32_t n = (uint32_t)leaves.size();
-        if (n >= kThreadLeaves)
-            leaf_thread_kernel<<<(n + 127) / 128, 128, 0, ctx.stream>>>((const LeafJob *)(d.p + o_leaves), n,
-                                                                        d.p + o_rows, (const uint32_t *)(d.p + o_widths),
-                                                                        pool);
-        else
-            leaf_kernel<<<(n * 32 + 127) / 128, 128, 0, ctx.stream>>>((const LeafJob *)(d.p + o_leaves), n,
-                                                                      d.p + o_rows, (const uint32_t *)(d.p + o_widths),
-                                                                      pool);
-        CK(cudaGetLastError());
-        ctx.launches++;
-    }
-    for (size_t l = 0; l + 1 < lv_off.size(); l++) {
-        const uint32_t n = (uint32_t)(lv_off[l + 1] - lv_off[l]);
-        if (!n) continue;
-        compress_kernel<<<(n * 32 + 127) / 128, 128, 0, ctx.stream>>>((const CJob *)(d.p + o_cj) + lv_off[l], n,
-                                                                      pool);
-        CK(cudaGetLastError());
-        ctx.launches++;
-    }
     for (size_t j = 0; j < nj; j++) {
         const Prepared &v = *act[j];
         const Plan &P = v.P;
@@ -846,9 +866,7 @@ inline void device_pass(Ctx &ctx, const std::vector<Prepared *> &vs, Timing *tm,
         da.bp = v.bp;
         da.de = de;
         da.flags = fl;
-        deep_kernel<<<(unsigned)((v.nq * 32 + 127) / 128), 128, 0, ctx.stream>>>(da);
-        CK(cudaGetLastError());
-        ctx.launches++;
+        das.push_back(da);
         if (!fri_shape_ok) continue;
         FriArgs fa{};
         fa.rows = d.p + o_rows;
@@ -869,7 +887,38 @@ inline void device_pass(Ctx &ctx, const std::vector<Prepared *> &vs, Timing *tm,
         fa.final_poly = d.p + o_fp[j];
         fa.final_deg = (uint32_t)v.final_deg;
         fa.flags = fl;
-        fri_kernel<<<1, 256, 0, ctx.stream>>>(fa);
+        fas.push_back(fa);
+    }
+    memcpy(st + o_das, das.data(), das.size() * sizeof(DeepArgs));
+    memcpy(st + o_fas, fas.data(), fas.size() * sizeof(FriArgs));
+    CK(cudaEventRecord(e0, ctx.stream));
+    ctx.h2d(d.p, st, staged);
+    ctx.h2d(pool + 4 * n_nodes, st + o_hints, hints.size());
+    CK(cudaMemsetAsync(back, 0, back_words * 8, ctx.stream));
+    if (!leaves.empty()) {
+        const uint32_t n = (uint32_t)leaves.size();
+        if (n >= kThreadLeaves)
+            leaf_thread_kernel<<<(n + 127) / 128, 128, 0, ctx.stream>>>((const LeafJob *)(d.p + o_leaves), n,
+                                                                        d.p + o_rows, (const uint32_t *)(d.p + o_widths),
+                                                                        pool);
+        else
+            leaf_kernel<<<(n * 32 + 127) / 128, 128, 0, ctx.stream>>>((const LeafJob *)(d.p + o_leaves), n,
+                                                                      d.p + o_rows, (const uint32_t *)(d.p + o_widths),
+                                                                      pool);
+        CK(cudaGetLastError());
+        ctx.launches++;
+    }
+    for (size_t l = 0; l + 1 < lv_off.size(); l++) {
+        launch_compress(ctx, (const CJob *)(d.p + o_cj) + lv_off[l], (uint32_t)(lv_off[l + 1] - lv_off[l]), pool);
+    }
+    if (!das.empty()) {
+        deep_kernel<<<dim3((unsigned)((max_nq * 32 + 127) / 128), (unsigned)das.size()), 128, 0, ctx.stream>>>(
+            (const DeepArgs *)(d.p + o_das));
+        CK(cudaGetLastError());
+        ctx.launches++;
+    }
+    if (!fas.empty()) {
+        fri_kernel<<<(unsigned)fas.size(), 256, 0, ctx.stream>>>((const FriArgs *)(d.p + o_fas));
         CK(cudaGetLastError());
         ctx.launches++;
     }
@@ -943,12 +992,7 @@ inline int lmcs_open_batch(Ctx &ctx, const uint64_t commit[4], const std::vector
         ctx.launches++;
     }
     for (size_t l = 0; l + 1 < lv_off.size(); l++) {
-        const uint32_t n = (uint32_t)(lv_off[l + 1] - lv_off[l]);
-        if (!n) continue;
-        compress_kernel<<<(n * 32 + 127) / 128, 128, 0, ctx.stream>>>((const CJob *)(d.p + o_cj) + lv_off[l], n,
-                                                                      pool);
-        CK(cudaGetLastError());
-        ctx.launches++;
+        launch_compress(ctx, (const CJob *)(d.p + o_cj) + lv_off[l], (uint32_t)(lv_off[l + 1] - lv_off[l]), pool);
     }
     uint64_t root[4] = {0, 0, 0, 0};
     if (!B.no_root) {
