@@ -396,14 +396,13 @@ P3G_API int p3g_fri_fold(p3g_ctx *x, const uint64_t *d_in, uint32_t log_n, uint3
         fa.w0inv = ntt::PowTab{tw.inv_lo.p, tw.inv_hi.p, tw.lo_bits};
         fa.beta = gl::ef{beta2[0], beta2[1]};
         fa.beta_dev = nullptr;
-        const uint64_t wi = gl::inv(gl::root(log_arity));
-        uint64_t w = 1;
-        for (int i = 0; i < 8; i++) fa.winv_a[i] = w, w = gl::mul(w, wi);
         fa.inv_a = gl::inv(1ull << log_arity);
         fa.out = d_out;
         fa.digests = nullptr;
-        const uint64_t threads = (fa.n_out + (1ull << log_arity) - 1) >> log_arity;
-        fri::fold_hash_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, x->c.stream>>>(fa);
+        const unsigned blocks = (unsigned)((fa.n_out + 127) / 128);
+        if (log_arity == 1) fri::fold_kernel<1><<<blocks, 128, 0, x->c.stream>>>(fa);
+        else if (log_arity == 2) fri::fold_kernel<2><<<blocks, 128, 0, x->c.stream>>>(fa);
+        else fri::fold_kernel<3><<<blocks, 128, 0, x->c.stream>>>(fa);
         CK(cudaGetLastError());
         x->c.launches++;
         x->c.sync();

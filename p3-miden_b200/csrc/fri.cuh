@@ -12,6 +12,7 @@
 // one leaf of the next tree.
 #pragma once
 #include "gl.cuh"
+#include "lde.cuh"
 #include "merkle.cuh"
 #include "ntt.cuh"
 
@@ -28,37 +29,47 @@ struct FoldArgs {
     ntt::PowTab w0inv;    // powers of w_{n0}^{-1}
     gl::ef beta;
     const uint64_t *beta_dev;  // if set, the challenge is read from here (device-side transcript)
-    uint64_t winv_a[8];   // w_a^{-t}, t < a
     uint64_t inv_a;       // 1/a
     uint64_t *out;        // n_out EF
     uint64_t *digests;    // (n_out / a) digests of the next round, or null
 };
 
+// Output k. The row holds y_t at bit-reversed positions, so the sums over t
+// are one decimation-in-time transform of each coordinate with the inverse
+// small roots (powers of two, lde.cuh): u_j = sum_t y_t w_a^{-jt}; then
+// Horner in beta/s. At arity 4 that is 8 sums and a shift per coordinate in
+// place of 16 products.
+template <int LA>
 __device__ __forceinline__ gl::ef fold_one(const FoldArgs &a, gl::ef beta, uint64_t k) {
-    const uint32_t A = 1u << a.log_a;
+    constexpr int A = 1 << LA;
     // s_inv = w_{n_in}^{-bitrev_{log n_out}(k)} = w_{n0}^{-(bitrev << (log n0 - log n_in))}
-    uint64_t e = gl::bitrev(k, a.log_nin - a.log_a) << (a.log_n0 - a.log_nin);
-    uint64_t s_inv = a.w0inv.at(e);
-    gl::ef x = gl::ef_mulf(beta, s_inv);
+    const uint64_t e = gl::bitrev(k, a.log_nin - LA) << (a.log_n0 - a.log_nin);
     const uint64_t *row = a.in + 2 * k * A;
-    if (A == 2) {
-        gl::ef y0{row[0], row[1]}, y1{row[2], row[3]};
-        gl::ef r = gl::ef_add(gl::ef_add(y0, y1), gl::ef_mul(gl::ef_sub(y0, y1), x));
-        return gl::ef_mulf(r, a.inv_a);
-    }
-    gl::ef y[8];
-    for (uint32_t t = 0; t < A; t++) {
-        uint64_t p = gl::bitrev(t, a.log_a);
-        y[t] = gl::ef{row[2 * p], row[2 * p + 1]};
-    }
-    gl::ef res = gl::ef_zero(), xp = gl::ef_one();
-    for (uint32_t j = 0; j < A; j++) {
-        gl::ef u = gl::ef_zero();
-        for (uint32_t t = 0; t < A; t++) u = gl::ef_add(u, gl::ef_mulf(y[t], a.winv_a[(j * t) & (A - 1)]));
-        res = gl::ef_add(res, gl::ef_mul(u, xp));
-        xp = gl::ef_mul(xp, x);
-    }
-    return gl::ef_mulf(res, a.inv_a);
+    uint64_t y0[A], y1[A];
+#pragma unroll
+    for (int p = 0; p < A; p++) y0[p] = row[2 * p], y1[p] = row[2 * p + 1];
+    const gl::ef x = gl::ef_mulf(beta, a.w0inv.at(e));
+    lde::dft_dit<LA>(y0);
+    lde::dft_dit<LA>(y1);
+    gl::ef r{y0[A - 1], y1[A - 1]};
+#pragma unroll
+    for (int j = A - 2; j >= 0; j--) r = gl::ef_add(gl::ef_mul(r, x), gl::ef{y0[j], y1[j]});
+    return gl::ef_mulf(r, a.inv_a);
+}
+__device__ __forceinline__ gl::ef fold_any(const FoldArgs &a, gl::ef beta, uint64_t k) {
+    return a.log_a == 1 ? fold_one<1>(a, beta, k) : a.log_a == 2 ? fold_one<2>(a, beta, k) : fold_one<3>(a, beta, k);
+}
+
+// The fold alone, one thread per output (2^20 values at arity 4: 44 us with
+// the row sums as products and four outputs per thread). Bound by latency and
+// launch below about 2^20 values, by the integer pipes above.
+template <int LA>
+__global__ void __launch_bounds__(128) fold_kernel(const __grid_constant__ FoldArgs a) {
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= a.n_out) return;
+    const gl::ef v = fold_one<LA>(a, a.beta, k);
+    a.out[2 * k] = v.c0;
+    a.out[2 * k + 1] = v.c1;
 }
 
 // thread g folds outputs [g*a, g*a + a)
@@ -70,7 +81,7 @@ __global__ void __launch_bounds__(128) fold_hash_kernel(const __grid_constant__ 
     const uint32_t cnt = (uint32_t)((a.n_out - g * A) < A ? (a.n_out - g * A) : A);
     const gl::ef beta = a.beta_dev ? gl::ef{a.beta_dev[0], a.beta_dev[1]} : a.beta;
     for (uint32_t u = 0; u < cnt; u++) {
-        gl::ef v = fold_one(a, beta, g * A + u);
+        gl::ef v = fold_any(a, beta, g * A + u);
         a.out[2 * (g * A + u)] = v.c0;
         a.out[2 * (g * A + u) + 1] = v.c1;
         buf[2 * u] = v.c0;
@@ -108,7 +119,7 @@ __global__ void __launch_bounds__(128) fold_hash_coop_kernel(const __grid_consta
     const gl::ef beta = a.beta_dev ? gl::ef{a.beta_dev[0], a.beta_dev[1]} : a.beta;
     uint64_t c0 = 0, c1 = 0;
     if ((uint32_t)l < cnt) {
-        const gl::ef v = fold_one(a, beta, g * A + l);
+        const gl::ef v = fold_any(a, beta, g * A + l);
         a.out[2 * (g * A + l)] = v.c0;
         a.out[2 * (g * A + l) + 1] = v.c1;
         c0 = v.c0, c1 = v.c1;

@@ -48,7 +48,7 @@ __device__ __forceinline__ uint64_t add_dev(uint64_t a, uint64_t b) {  // a, b <
         : "r"((uint32_t)a), "r"((uint32_t)(a >> 32)), "r"((uint32_t)b), "r"((uint32_t)(b >> 32)));
     return ((uint64_t)r1 << 32) | r0;
 }
-// b < p: a - b mod p, below p when a < p, below 2^64 (weak) when a < 2^64
+// b <= p (p counts as 0): a - b mod p, below p when a < p, below 2^64 (weak) when a < 2^64
 __device__ __forceinline__ uint64_t sub_dev(uint64_t a, uint64_t b) {
     uint32_t r0, r1;
     asm("{\n\t.reg .u32 m;\n\t"

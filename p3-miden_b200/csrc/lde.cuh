@@ -48,7 +48,9 @@
 namespace lde {
 
 // a + b as a - (p - b): seven instructions against nine for add_dev (p - b
-// = p when b = 0; the borrow then adds p back)
+// = p when b = 0; the borrow then adds p back). add_dev stays where it is the
+// faster one: the generated constraint kernels took 25.5 ms with this form,
+// 18.7 with add_dev (2^18-row Keccak proof).
 __device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) { return gl::sub_dev(a, gl::P - b); }
 __device__ __forceinline__ uint64_t sub(uint64_t a, uint64_t b) { return gl::sub_dev(a, b); }
 // a times the word whose Montgomery form is m

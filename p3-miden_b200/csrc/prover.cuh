@@ -875,11 +875,6 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
             next_tree = std::move(t);
         }
     }
-    uint64_t winv_a[8];
-    {
-        uint64_t wi = gl::inv(gl::root(log_a)), x = 1;
-        for (uint64_t t = 0; t < 8; t++) winv_a[t] = x, x = gl::mul(x, wi);
-    }
     // The rounds run without host round trips: the challenger lives on the
     // device for the loop (fri::DevCh). Per round: observe the root, grind,
     // check the witness and sample beta (one-thread kernels), fold + hash the
@@ -931,7 +926,6 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
         fa.log_n0 = log_lde;
         fa.w0inv = ntt::PowTab{tw0.inv_lo.p, tw0.inv_hi.p, tw0.lo_bits};
         fa.beta_dev = dbeta.p + 2 * r;
-        memcpy(fa.winv_a, winv_a, sizeof(winv_a));
         fa.inv_a = gl::inv(arity);
         fa.out = out.p;
         bool more = nout > final_dom;
