@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const uint64_t *M, uint64_t
     const uint64_t col = (uint64_t)blockIdx.x * 32 + cl;
     const uint64_t r0 = (uint64_t)blockIdx.y * rows_per_chunk;
     const uint64_t r1 = min(d, r0 + rows_per_chunk);
-    gl::Acc acc[4];
+    gl::SplitAcc acc[4];
     if (col < w) {
         // four rows per step: their loads are issued together, so that each
         // thread keeps several DRAM reads in flight
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(256) rowdot_lanes_kernel(const uint64_t *M, ui
     for (uint64_t base = first - (threadIdx.x % 32) / G; base < h; base += rows) {
         const uint64_t i = base + (threadIdx.x % 32) / G;
         const uint64_t *row = M + (i < h ? i : h - 1) * w;
-        gl::Acc a0, a1;
+        gl::SplitAcc a0, a1;
         for (uint64_t col = lane; col < padded; col += 4 * G) {  // four loads in flight per lane
             uint64_t v[4];
 #pragma unroll
@@ -271,7 +271,7 @@ __global__ void rowdot_thread_kernel(const uint64_t *M, uint64_t h, uint64_t w, 
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= h) return;
     const uint64_t *row = M + i * w;
-    gl::Acc a0, a1;
+    gl::SplitAcc a0, a1;
     for (uint64_t col = 0; col < w; col++) {
         uint64_t v = __ldg(row + col);
         a0.mac(v, __ldg(coef + 2 * col));
