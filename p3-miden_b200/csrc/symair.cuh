@@ -76,6 +76,11 @@ struct KLayout {
     uint64_t pub = 0, rnd = 0, auxv = 0, alpha = 0, words = 0;
 };
 
+// Constraints evaluated together: `step` in step with one another, `small`
+// as soon as their cells are loaded (indices into Desc::constraints).
+struct ChunkGroup {
+    std::vector<uint32_t> step, small;
+};
 struct Air {
     Desc d;
     std::vector<uint32_t> degree;   // per node
@@ -84,7 +89,7 @@ struct Air {
     bool uses_first = false, uses_last = false, uses_trans = false;
     std::vector<uint64_t> base_idx, ext_idx;  // ConstraintLayout
     KLayout kl;
-    std::vector<std::vector<uint32_t>> chunks;  // constraint indices of each generated kernel
+    std::vector<std::vector<ChunkGroup>> chunks;  // constraints of each generated kernel
     size_t chunk_nodes = 500;  // DAG nodes per chunk (a launch-shape choice; every value gives the same sums)
     std::string source, log;
     std::vector<std::vector<char>> cubins;  // one per compiled group of chunks
@@ -209,46 +214,151 @@ struct KArgs {
     uint64_t *acc;         // EF accumulator, += the folded numerator
 };
 
-// Constraints are split into chunks of bounded code size (at most
+// Constraints are split into chunks of bounded code size (about
 // A.chunk_nodes DAG nodes each, shared subexpressions counted once per chunk);
 // each chunk is one kernel that adds its part of the fold into acc. The fold
 // is linear, so launching the chunks one after another on the same stream
-// gives the same sum. A small AIR is one chunk.
+// gives the same sum, in any order of the constraints. A small AIR is one
+// chunk.
+//
+// A cell that two chunks read is loaded from HBM twice, and a subexpression
+// two chunks need is evaluated twice, so constraints are first grouped by what
+// they share: a group is up to kGroupMax constraints of similar size that
+// share at least a quarter of their nodes with it (the Keccak AIR's limbs of
+// one column over the five planes; its chi limbs of one plane), evaluated in
+// step, node by node, so that a shared value is used by all of them while it
+// is live; and the small constraints (booleans, parities) whose cells a group
+// loads follow as soon as their last cell is there. In emission order the
+// Keccak AIR's chunks loaded 14.6 k cells per point, 5.5 times its columns.
+constexpr size_t kGroupMax = 5, kSmallNodes = 40;
 
 inline void split_chunks(Air &A) {
     const Desc &d = A.d;
-    const size_t n = d.nodes.size();
-    A.chunks.assign(1, {});
-    std::vector<uint32_t> owner(n, 0), seen(n, 0), st, walk;
-    uint32_t cid = 1, epoch = 0;
-    size_t in_chunk = 0;
-    // the nodes under `root` that the current chunk does not hold yet
-    auto collect = [&](uint32_t root) {
-        walk.clear();
-        st.assign(1, root);
-        ++epoch;
+    const size_t n = d.nodes.size(), nc = d.constraints.size();
+    auto binary = [](const Node &x) { return x.op == ADD || x.op == SUB || x.op == MUL; };
+    auto is_cell = [](const Node &x) { return x.op == MAIN || x.op == AUX; };
+    // each constraint's nodes (constants and other scalars left out)
+    std::vector<std::vector<uint32_t>> nodes(nc);
+    std::vector<uint32_t> seen(n, 0), st;
+    for (size_t k = 0; k < nc; k++) {
+        st.assign(1, d.constraints[k]);
         while (!st.empty()) {
             const uint32_t i = st.back();
             st.pop_back();
-            if (owner[i] == cid || seen[i] == epoch) continue;
-            seen[i] = epoch;
-            walk.push_back(i);
+            if (seen[i] == k + 1) continue;
+            seen[i] = (uint32_t)k + 1;
             const Node &x = d.nodes[i];
-            if (x.op == ADD || x.op == SUB || x.op == MUL) st.push_back(x.a), st.push_back(x.b);
-            if (x.op == NEG) st.push_back(x.a);
+            if (binary(x)) st.push_back(x.a), st.push_back(x.b);
+            else if (x.op == NEG) st.push_back(x.a);
+            else if (!is_cell(x)) continue;
+            nodes[k].push_back(i);
         }
+    }
+    // readers of each node among the larger constraints; a node most of them
+    // read says nothing
+    std::vector<std::vector<uint32_t>> readers(n);
+    for (size_t k = 0; k < nc; k++)
+        if (nodes[k].size() > kSmallNodes)
+            for (uint32_t i : nodes[k]) readers[i].push_back((uint32_t)k);
+    constexpr size_t kCommon = 64;
+    // a cell counts twice: it is a load as well as a node
+    auto weight = [&](uint32_t i) -> uint32_t { return is_cell(d.nodes[i]) ? 2 : 1; };
+    std::vector<uint32_t> size(nc, 0);
+    for (size_t k = 0; k < nc; k++)
+        for (uint32_t i : nodes[k]) size[k] += weight(i);
+    std::vector<uint8_t> placed(nc, 0);
+    std::vector<ChunkGroup> groups;
+    std::vector<uint32_t> shared(nc, 0), touched;
+    for (size_t k = 0; k < nc; k++) {
+        if (placed[k] || nodes[k].size() <= kSmallNodes) continue;
+        ChunkGroup g;
+        touched.clear();
+        uint32_t add = (uint32_t)k;
+        for (;;) {
+            g.step.push_back(add);
+            placed[add] = 1;
+            for (uint32_t i : nodes[add]) {
+                if (seen[i] == nc + 1 + k) continue;  // counted for this group
+                seen[i] = (uint32_t)(nc + 1 + k);
+                if (readers[i].size() > kCommon) continue;
+                for (uint32_t u : readers[i]) {
+                    if (placed[u]) continue;
+                    if (!shared[u]) touched.push_back(u);
+                    shared[u] += weight(i);
+                }
+            }
+            if (g.step.size() == kGroupMax) break;
+            int64_t best = -1;
+            for (uint32_t u : touched)
+                if (!placed[u] && 4 * shared[u] >= size[u] && size[u] <= 2 * size[k] && size[k] <= 2 * size[u] &&
+                    (best < 0 || shared[u] > shared[best] || (shared[u] == shared[best] && u < best)))
+                    best = u;
+            if (best < 0) break;
+            add = (uint32_t)best;
+        }
+        for (uint32_t u : touched) shared[u] = 0;
+        groups.push_back(std::move(g));
+    }
+    // small constraints: to the first group that loads all their cells
+    std::vector<int64_t> cell_group(n, -1);  // last group seen loading the cell
+    std::vector<std::vector<uint32_t>> cell_groups(n);
+    for (size_t g = 0; g < groups.size(); g++)
+        for (uint32_t k : groups[g].step)
+            for (uint32_t i : nodes[k])
+                if (is_cell(d.nodes[i]) && cell_group[i] != (int64_t)g)
+                    cell_group[i] = (int64_t)g, cell_groups[i].push_back((uint32_t)g);
+    std::vector<uint32_t> hits(groups.size(), 0);
+    std::vector<ChunkGroup> rest;
+    for (size_t k = 0; k < nc; k++) {
+        if (placed[k]) continue;
+        size_t cells = 0;
+        int64_t home = -1;
+        touched.clear();
+        for (uint32_t i : nodes[k])
+            if (is_cell(d.nodes[i])) {
+                cells++;
+                if (cell_groups[i].size() > kCommon) continue;
+                for (uint32_t g : cell_groups[i])
+                    if (hits[g]++ == 0) touched.push_back(g);
+            }
+        for (uint32_t g : touched) {
+            if (cells && hits[g] == cells && (home < 0 || g < home)) home = g;
+            hits[g] = 0;
+        }
+        if (home >= 0) {
+            groups[home].small.push_back((uint32_t)k);
+        } else {
+            rest.emplace_back();
+            rest.back().step.push_back((uint32_t)k);
+        }
+    }
+    for (ChunkGroup &g : rest) groups.push_back(std::move(g));
+    // chunks of whole groups
+    A.chunks.assign(1, {});
+    std::vector<uint32_t> owner(n, 0);
+    uint32_t cid = 1;
+    size_t in_chunk = 0;
+    std::vector<uint32_t> fresh;
+    auto collect = [&](const ChunkGroup &g) {  // nodes of g the current chunk does not hold yet
+        fresh.clear();
+        for (const auto *v : {&g.step, &g.small})
+            for (uint32_t k : *v)
+                for (uint32_t i : nodes[k])
+                    if (owner[i] != cid) fresh.push_back(i);
+        std::sort(fresh.begin(), fresh.end());
+        fresh.erase(std::unique(fresh.begin(), fresh.end()), fresh.end());
     };
-    for (size_t k = 0; k < d.constraints.size(); k++) {
-        collect(d.constraints[k]);
-        if (!A.chunks.back().empty() && in_chunk + walk.size() > A.chunk_nodes) {
+    for (ChunkGroup &g : groups) {
+        collect(g);
+        if (!A.chunks.back().empty() && in_chunk + fresh.size() > A.chunk_nodes) {
             A.chunks.emplace_back();
             cid++;
             in_chunk = 0;
-            collect(d.constraints[k]);
+            collect(g);
         }
-        for (uint32_t i : walk) owner[i] = cid;
-        in_chunk += walk.size();
-        A.chunks.back().push_back((uint32_t)k);
+        for (uint32_t i : fresh) owner[i] = cid;
+        in_chunk += fresh.size();
+        A.chunks.back().push_back(std::move(g));
     }
 }
 
@@ -324,9 +434,11 @@ struct KArgs {
         inner[i] = linear[i] && !is_root[i] && reader[i] >= 0 && linear[reader[i]];
     std::vector<uint8_t> live(n);
     for (size_t c = c0; c < c1; c++) {
-        const std::vector<uint32_t> &ks = A.chunks[c];
+        const std::vector<ChunkGroup> &gs = A.chunks[c];
         std::fill(live.begin(), live.end(), 0);
-        for (uint32_t k : ks) live[d.constraints[k]] = 1;
+        for (const ChunkGroup &g : gs)
+            for (const auto *v : {&g.step, &g.small})
+                for (uint32_t k : *v) live[d.constraints[k]] = 1;
         bool first = false, last = false, trans = false;
         for (size_t i = n; i-- > 0;) {
             if (!live[i]) continue;
@@ -360,14 +472,17 @@ struct KArgs {
             if (last) o << "    const uint64_t s_last = gl::mul(zh, gl::inv(gl::sub(x, a.omega_h_inv)));\n";
             if (trans) o << "    const uint64_t s_trans = gl::sub(x, a.omega_h_inv);\n";
         }
-        // constraint by constraint: the nodes of its expression not emitted
-        // yet, in post-order (each load just before its first use), then its
-        // term of the fold, so that a value lives only while a later node of
-        // the chunk still reads it (register pressure sets the occupancy of
-        // these long straight-line kernels). Base constraints go into two lazy
-        // accumulators (one per coordinate of alpha^{K-1-k}), extension
-        // constraints into an extension sum.
+        // group by group: the nodes of its constraints not emitted yet, each
+        // constraint's in post-order (each load just before its first use) and
+        // the constraints of a group in step, then each one's term of the
+        // fold, so that a value lives only while a nearby node still reads it
+        // (register pressure sets the occupancy of these long straight-line
+        // kernels). Base constraints go into two lazy accumulators (one per
+        // coordinate of alpha^{K-1-k}), extension constraints into an
+        // extension sum.
         std::vector<uint8_t> done(n, 0);
+        std::vector<uint32_t> mark(n, 0);
+        uint32_t epoch = 0;
         std::vector<std::pair<uint32_t, bool>> st;
         std::vector<uint8_t> bits(n, 64);
         // a multiple of p at or above 2^b (64 <= b <= 95), as "lo, hi"
@@ -460,13 +575,15 @@ struct KArgs {
             o << ";\n";
         };
         o << "    gl::Acc f0, f1;\n    gl::ef fe = gl::ef_zero();\n";
-        for (uint32_t k : ks) {
-            const uint32_t cn = d.constraints[k];
-            st.assign(1, {cn, false});
-            while (!st.empty()) {  // iterative post-order over the nodes not emitted yet
+        // a constraint's nodes in post-order (fused sums left out)
+        auto post_order = [&](uint32_t root, std::vector<uint32_t> &seq) {
+            seq.clear();
+            epoch++;
+            st.assign(1, {root, false});
+            while (!st.empty()) {
                 const auto [i, expanded] = st.back();
                 st.pop_back();
-                if (done[i]) continue;
+                if (done[i] || mark[i] == epoch) continue;
                 const Node &x = d.nodes[i];
                 const bool binary = x.op == ADD || x.op == SUB || x.op == MUL;
                 if (!expanded && (binary || x.op == NEG)) {
@@ -481,9 +598,12 @@ struct KArgs {
                     st.push_back({x.a, false});
                     continue;
                 }
-                done[i] = 1;
-                emit_node(i);
+                mark[i] = epoch;
+                seq.push_back(i);
             }
+        };
+        auto emit_fold = [&](uint32_t k) {
+            const uint32_t cn = d.constraints[k];
             const uint64_t ap = A.kl.alpha + 2ull * k;
             if (!A.ext[cn])
                 o << "    f0.mac(v" << cn << ", __ldg(K + " << ap << ")); f1.mac(v" << cn << ", __ldg(K + " << ap + 1
@@ -491,6 +611,52 @@ struct KArgs {
             else
                 o << "    fe = gl::ef_add(fe, gl::ef_mul(v" << cn << ", gl::ef{__ldg(K + " << ap << "), __ldg(K + "
                   << ap + 1 << ")}));\n";
+        };
+        std::vector<uint32_t> seq;
+        auto emit_whole = [&](uint32_t k) {
+            post_order(d.constraints[k], seq);
+            for (uint32_t i : seq) done[i] = 1, emit_node(i);
+            emit_fold(k);
+        };
+        for (const ChunkGroup &g : gs) {
+            // the small constraints waiting for a cell
+            std::vector<uint32_t> missing(g.small.size(), 0);
+            std::map<uint32_t, std::vector<uint32_t>> by_cell;
+            for (size_t q = 0; q < g.small.size(); q++) {
+                post_order(d.constraints[g.small[q]], seq);
+                for (uint32_t i : seq)
+                    if (d.nodes[i].op == MAIN || d.nodes[i].op == AUX) by_cell[i].push_back((uint32_t)q), missing[q]++;
+            }
+            std::vector<uint8_t> out(g.small.size(), 0);
+            auto emit_ready = [&](uint32_t q) {
+                if (!out[q]) out[q] = 1, emit_whole(g.small[q]);
+            };
+            for (size_t q = 0; q < g.small.size(); q++)
+                if (!missing[q]) emit_ready((uint32_t)q);
+            std::vector<std::vector<uint32_t>> seqs(g.step.size());
+            std::vector<size_t> at(g.step.size(), 0);
+            for (size_t q = 0; q < g.step.size(); q++) post_order(d.constraints[g.step[q]], seqs[q]);
+            for (;;) {  // the constraint least far through its nodes goes next
+                int64_t best = -1;
+                for (size_t q = 0; q < seqs.size(); q++)
+                    if (at[q] < seqs[q].size() &&
+                        (best < 0 || at[q] * seqs[best].size() < at[best] * seqs[q].size()))
+                        best = (int64_t)q;
+                if (best < 0) break;
+                const uint32_t i = seqs[best][at[best]++];
+                if (!done[i]) {
+                    done[i] = 1;
+                    emit_node(i);
+                    auto w = by_cell.find(i);
+                    if (w != by_cell.end())
+                        for (uint32_t q : w->second)
+                            if (--missing[q] == 0) emit_ready(q);
+                }
+                if (at[best] == seqs[best].size()) emit_fold(g.step[best]);
+            }
+            for (size_t q = 0; q < g.step.size(); q++)
+                if (seqs[q].empty()) emit_fold(g.step[q]);  // its root was already there
+            for (size_t q = 0; q < g.small.size(); q++) emit_ready((uint32_t)q);
         }
         o << R"K(    const gl::ef r = gl::ef_add(gl::ef{f0.reduce(), f1.reduce()}, fe);
     uint64_t *out = a.acc + 2 * m;
