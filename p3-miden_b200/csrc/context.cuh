@@ -698,11 +698,12 @@ inline void launch_tc(Ctx &ctx, std::atomic<uint64_t> &attr_done, K kernel, uint
 }
 
 // Leaf sponge of one height class of n leaves, by how many lanes fill the
-// chip: 16 per leaf up to 2^11 leaves (latency-bound), four for 2^12 and 2^13,
-// one for 2^14, and the tensor-core permutation from 2^15 on (the figures
-// are at leaf_class_quad_kernel; 2^15 leaves x 512 columns with four lanes
-// each take 2.9 ms against 2.4, 2^16 5.2 against 3.3).
-constexpr uint64_t kTcLeaves = 1ull << 15, kQuadLeaves = 1ull << 13;
+// chip: 16 per leaf up to 2^11 leaves (latency-bound), four for 2^12 to 2^14,
+// and the tensor-core permutation from 2^15 on, or one thread per leaf where
+// the constants do not fit its byte tables (the figures are at
+// leaf_class_quad_kernel; 2^15 / 2^16 leaves x 512 columns take 2.35 / 3.23 ms
+// on the tensor cores, 2.55 / 4.76 with four lanes, 2.37 / 4.18 with one).
+constexpr uint64_t kTcLeaves = 1ull << 15, kQuadLeaves = 1ull << 14;
 inline void launch_leaf_class(Ctx &ctx, const merkle::ClassArgs &a, uint64_t n) {
     const unsigned coop_blocks = (unsigned)((n * 16 + 127) / 128), blocks = (unsigned)((n + 127) / 128);
     if (a.cm && a.n_mats != 1) throw CudaError{ERR_INVALID, "column-major copy of a multi-matrix class"};

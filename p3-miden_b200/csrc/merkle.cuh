@@ -213,15 +213,19 @@ __device__ __forceinline__ void p2_permute_dev(uint64_t *s) {
 
 
 // Permutation shared by 16 lanes, for latency-bound work (a few states at a
-// time; about a third of the single-thread latency). Lane l < 12 holds word
+// time; about 0.28 of the single-thread latency). Lane l < 12 holds word
 // l, lanes 12..15 hold zero between rounds. External rounds run one S-box per
 // lane and move the M4 and cross-block sums through shuffles. In the internal
 // rounds every lane carries a copy z of s_0: the S-box runs on z while the
 // sum R of s_1..s_11 is formed by a 4-step butterfly, and
-// s_0 <- (mu_0 + 1) * S(z) + R, so only the S-box and one product lie on the
-// round's critical path. Same lazy arithmetic as p2_permute_dev (results
-// agree mod p); the diagonal products take the plain reduction, whose 96-bit
-// addend needs no reduction of its own. Two states per warp; all 32 lanes must call it. `sc` is the
+// s_0 <- (mu_0 + 1) * S(z) + R, s_i <- mu_i s_i + R + S(z) are one product in
+// every lane, with the next round's constant in lane 0's sum; lane 0's word is
+// then broadcast. A lone warp is bound by its own issue as much as by the
+// chain, so the shared product pays for the broadcast: a chained permutation
+// takes 12.8 k cycles, 17.0 k with a second product for z in every lane. Same
+// lazy arithmetic as p2_permute_dev (results agree mod p); the diagonal
+// products take the plain reduction, whose 96-bit addend needs no reduction of
+// its own. Two states per warp; all 32 lanes must call it. `sc` is the
 // constant table staged in shared memory (stage_consts).
 namespace p2x {
 // copy the constant table into shared memory (all threads of the block call it)
@@ -234,36 +238,37 @@ __device__ __forceinline__ uint64_t shfl64(uint64_t v, int src) {
     const uint32_t hi = __shfl_sync(0xffffffffu, (uint32_t)(v >> 32), src, 16);
     return ((uint64_t)hi << 32) | lo;
 }
-__device__ __forceinline__ p2w::W shflW(p2w::W v, int src) {
-    return p2w::W{shfl64(v.lo, src), __shfl_sync(0xffffffffu, v.hi, src, 16)};
-}
 __device__ __forceinline__ p2w::W shflW_xor(p2w::W v, int m) {
     const uint32_t lo = __shfl_xor_sync(0xffffffffu, (uint32_t)v.lo, m, 16);
     const uint32_t hi = __shfl_xor_sync(0xffffffffu, (uint32_t)(v.lo >> 32), m, 16);
     return p2w::W{((uint64_t)hi << 32) | lo, __shfl_xor_sync(0xffffffffu, v.hi, m, 16)};
 }
 struct Lane {
-    uint64_t mu;     // diagonal word l (0 for l >= 12)
-    uint64_t mu0p1;  // mu_0 + 1 mod p
+    uint64_t mu;  // diagonal word l; mu_0 + 1 mod p in lane 0; 0 for l >= 12
 };
 __device__ __forceinline__ Lane lane_consts(const uint64_t *sc, int l) {
-    return Lane{l < 12 ? sc[p2::OFF_DIAG + l] : 0, gl::add_dev(sc[p2::OFF_DIAG], 1)};
+    return Lane{l == 0 ? gl::add_dev(sc[p2::OFF_DIAG], 1) : l < 12 ? sc[p2::OFF_DIAG + l] : 0};
 }
-// circ(2*M4, M4, M4) for word l: M4 row (l mod 4) of its block, plus the sum
-// over the three blocks of that row; lanes 12..15 return 0
-// rc: the lane's constant of the next round (0 for none), added to the
-// 96-bit sum before the reduction
+// circ(2*M4, M4, M4) for word l: M4 of v = x_l + the sum of the three blocks'
+// words at position l mod 4, with sums modulo 2^64 beside those of the top 27
+// bits as in p2w::ext_linear (28 words in all). rc: the lane's constant of the
+// next round (0 for none). Lanes 12..15 return values nobody reads.
 __device__ __forceinline__ uint64_t ext_linear(uint64_t x, int l, uint64_t rc = 0) {
-    using namespace p2w;
-    const int base = l & ~3, j = l & 3;
-    const uint64_t x0 = shfl64(x, base), x1 = shfl64(x, base + 1), x2 = shfl64(x, base + 2), x3 = shfl64(x, base + 3);
-    const W t01 = wadd1(wide(x0), x1), t23 = wadd1(wide(x2), x3);
-    const W t0123 = wadd(t01, t23);
-    const uint64_t e = j < 2 ? x1 : x3;
-    const W f = j == 0 ? t01 : j == 1 ? wdbl(x2) : j == 2 ? t23 : wdbl(x0);
-    const W y = wadd(wadd1(t0123, e), f);
-    const W t = wadd(wadd(shflW(y, j), shflW(y, j + 4)), shflW(y, j + 8));
-    return l < 12 ? wreduce(wadd1(wadd(y, t), rc)) : 0;
+    const uint64_t xa = shfl64(x, l < 8 ? l + 4 : l - 8), xb = shfl64(x, l < 4 ? l + 8 : l - 4);
+    const uint64_t v = x + x + xa + xb;
+    const uint32_t h = 2 * (uint32_t)(x >> 37) + (uint32_t)(xa >> 37) + (uint32_t)(xb >> 37);
+    const int base = l & ~3;
+    uint64_t w = v + v + rc;
+    uint32_t u = h + h + (uint32_t)(rc >> 37);
+#pragma unroll
+    for (int d = 1; d < 4; d++) {
+        const int src = base | ((l + d) & 3);
+        const uint64_t vd = shfl64(v, src);
+        const uint32_t hd = __shfl_sync(0xffffffffu, h, src, 16);
+        w += d == 1 ? vd + vd + vd : vd;
+        u += d == 1 ? 3 * hd : hd;
+    }
+    return p2w::fold_wraps(w, u);
 }
 // four external rounds whose first constant is already in x; each linear
 // layer takes in the next round's constant
@@ -277,18 +282,16 @@ __device__ __forceinline__ uint64_t permute(uint64_t x, int l, const uint64_t *s
     using namespace p2w;
     const int li = l < 12 ? l : 11;
     x = ext_rounds(ext_linear(x, l, sc[p2::OFF_INIT + li]), l, sc + p2::OFF_INIT);
-    uint64_t z = shfl64(x, 0);
-    const bool rest = l >= 1 && l < 12;
+    const bool first = l == 0, rest = l >= 1 && l < 12;
+    if (first) x = add_c(x, sc[p2::OFF_INT]);
 #pragma unroll 1
     for (int r = 0; r < 22; r++) {
-        const uint64_t zs = sbox(add_c(z, sc[p2::OFF_INT + r]));
+        const uint64_t zs = sbox(shfl64(x, 0)), rc = r < 21 ? sc[p2::OFF_INT + r + 1] : 0;
         W P = wide(rest ? x : 0);
 #pragma unroll
         for (int m = 1; m < 16; m <<= 1) P = wadd(P, shflW_xor(P, m));
-        z = mul_add_w(zs, k.mu0p1, P);                       // P < 11 * 2^64
-        x = rest ? mul_add_w(x, k.mu, wadd1(P, zs)) : 0;     // sum < 12 * 2^64
+        x = mul_add_w(first ? zs : x, k.mu, wadd1(P, first ? rc : zs));  // sum < 12 * 2^64
     }
-    if (l == 0) x = z;
     return ext_rounds(add_c(x, sc[p2::OFF_TERM + li]), l, sc + p2::OFF_TERM);
 }
 }  // namespace p2x
@@ -299,7 +302,7 @@ __device__ __forceinline__ uint64_t permute(uint64_t x, int l, const uint64_t *s
 // one exchange of the four positions, y_l = 2 v_l + 3 v_{l+1} + v_{l+2} +
 // v_{l+3}. Internal rounds as p2x::permute. About 800 warp instructions per
 // state against 545 for one thread per state and 2450 for 16 lanes; alone, a
-// chained permutation takes 22.0 k cycles against 44.9 and 17.0. 8 states per
+// chained permutation takes 17.7 k cycles against 44.9 and 12.8. 8 states per
 // warp; all 32 lanes must call it. `sc`: p2x::stage_consts.
 namespace p2q {
 __device__ __forceinline__ uint32_t from(uint32_t v, int d) {  // lane l + d of the quad
@@ -333,12 +336,11 @@ __device__ __forceinline__ void ext_linear(uint64_t *x, const uint64_t *sc, int 
     }
 }
 struct Lane {
-    uint64_t mu[3];   // diagonal words of the lane (0 for word 0)
-    uint64_t mu0p1;   // mu_0 + 1 mod p
+    uint64_t mu[3];  // diagonal words of the lane; mu_0 + 1 mod p for word 0
 };
 __device__ __forceinline__ Lane lane_consts(const uint64_t *sc, int l) {
-    return Lane{{l ? sc[p2::OFF_DIAG + l] : 0, sc[p2::OFF_DIAG + l + 4], sc[p2::OFF_DIAG + l + 8]},
-                gl::add_dev(sc[p2::OFF_DIAG], 1)};
+    return Lane{{l ? sc[p2::OFF_DIAG + l] : gl::add_dev(sc[p2::OFF_DIAG], 1), sc[p2::OFF_DIAG + l + 4],
+                 sc[p2::OFF_DIAG + l + 8]}};
 }
 __device__ __forceinline__ void permute(uint64_t *x, const uint64_t *sc, const Lane &k) {
     using namespace p2w;
@@ -347,22 +349,20 @@ __device__ __forceinline__ void permute(uint64_t *x, const uint64_t *sc, const L
 #pragma unroll 1
     for (int r = 0; r < 8; r++) {
         if (r == 4) {
-            uint64_t z = ((uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(x[0] >> 32), 0, 4) << 32) |
-                         __shfl_sync(0xffffffffu, (uint32_t)x[0], 0, 4);
-            if (l == 0) x[0] = 0;
+            if (l == 0) x[0] = add_c(x[0], sc[p2::OFF_INT]);
 #pragma unroll 1
             for (int q = 0; q < 22; q++) {
-                const uint64_t zs = sbox(add_c(z, sc[p2::OFF_INT + q]));
-                W P = wadd1(wadd1(wide(x[0]), x[1]), x[2]);
+                const uint64_t z = ((uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(x[0] >> 32), 0, 4) << 32) |
+                                   __shfl_sync(0xffffffffu, (uint32_t)x[0], 0, 4);
+                const uint64_t zs = sbox(z), rc = q < 21 ? sc[p2::OFF_INT + q + 1] : 0;
+                W P = wadd1(wadd1(wide(l ? x[0] : 0), x[1]), x[2]);
 #pragma unroll
                 for (int m = 1; m < 4; m <<= 1) P = wadd(P, p2x::shflW_xor(P, m));
-                z = mul_add_w(zs, k.mu0p1, P);  // P < 11 * 2^64
-                const W t = wadd1(P, zs);       // < 12 * 2^64
-                x[0] = l ? mul_add_w(x[0], k.mu[0], t) : 0;
+                const W t = wadd1(P, zs);  // < 12 * 2^64
+                x[0] = mul_add_w(l ? x[0] : zs, k.mu[0], l ? t : wadd1(P, rc));
                 x[1] = mul_add_w(x[1], k.mu[1], t);
                 x[2] = mul_add_w(x[2], k.mu[2], t);
             }
-            if (l == 0) x[0] = z;
 #pragma unroll
             for (int i = 0; i < 3; i++) x[i] = add_c(x[i], sc[p2::OFF_TERM + l + 4 * i]);
         }
@@ -487,13 +487,13 @@ __global__ void __launch_bounds__(128) leaf_class_coop_kernel(const __grid_const
     }
 }
 
-// The leaf sponge with four lanes per leaf (p2q), for classes of 2^12 and
-// 2^13 leaves: one thread per leaf leaves most schedulers without a warp
-// there, and 16 lanes per leaf more than fill them. Trees of 2^11 / 2^12 /
-// 2^13 / 2^14 leaves x 512 columns took 0.88 / 1.25 / 1.96 / 3.51 ms with 16
-// lanes, 0.93 / 0.94 / 1.15 / 1.85 with four and - / - / 1.68 / 1.72 with one
-// thread. The next chunk's words are loaded before the permutation of this
-// one.
+// The leaf sponge with four lanes per leaf (p2q), for classes of 2^12 to 2^14
+// leaves: one thread per leaf leaves most schedulers without a warp there, and
+// 16 lanes per leaf more than fill them. Trees of 2^11 / 2^12 / 2^13 / 2^14 /
+// 2^15 leaves x 512 columns took 0.69 / 1.05 / 1.63 / 2.96 / 5.61 ms with 16
+// lanes, - / 0.70 / 0.93 / 1.59 / 2.55 with four and 1.59 / 1.62 / 1.64 / 1.65
+// / 2.37 with one thread. The next chunk's words are loaded before the
+// permutation of this one.
 template <bool CM>
 __global__ void __launch_bounds__(128) leaf_class_quad_kernel(const __grid_constant__ ClassArgs a) {
     __shared__ uint64_t sc[p2::N_PARAMS];

@@ -27,7 +27,7 @@ CASES = [
     ([(1 << 12, 17)], 8, "edges"),                       # four lanes per leaf
     ([(1 << 9, 4), (1 << 12, 8), (1 << 13, 13), (1 << 13, 1)], 8, "random"),  # carried states, two matrices
     ([(1 << 13, 3)], 1, "top"),
-    ([(1 << 14, 12)], 8, "edges"),                       # one thread per leaf
+    ([(1 << 14, 12)], 8, "edges"),                       # the last class of four lanes per leaf
     ([(1 << 15, 1)], 1, "random"),                       # two groups per SM, one short chunk
     ([(1 << 15, 8)], 8, "top"),
     ([(1 << 15, 9)], 8, "edges"),                        # a chunk and one word
