@@ -245,12 +245,32 @@ struct GrindArgs {
     unsigned long long *found;  // atomicMin target, initialised to ~0
     const DevCh *ch;            // if set, state and pending inputs are read from this device challenger
 };
+// A witness below every one this thread could still find is there: the word
+// is asked for a round ahead of its use (it lies in L2).
+struct WitnessFound {
+    const volatile unsigned long long *found;
+    uint64_t w, seen;
+    __device__ __forceinline__ bool operator()() {
+        const bool stop = w >= seen;
+        seen = *found;
+        return stop;
+    }
+};
+// Candidates are tried in order, a grid's worth at a time, so that the least
+// witness is found. Bound by the latency of a permutation and its integer
+// pipes. Two blocks per SM: a turn of 38 k candidates takes 36 us, and more
+// blocks try more candidates past the least witness (16 bits, mean of 300
+// states with the call: 1 / 2 / 3 / 4 / 8 blocks 133 / 109 / 115 / 125 / 158
+// us; 130 us with two when a turn begun beside the find ran to its end).
+constexpr int kGrindBlocks = 2;
 __global__ void __launch_bounds__(128) grind_kernel(const __grid_constant__ GrindArgs a) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t mask = (1ull << a.bits) - 1;
+    WitnessFound stop{a.found, 0, ~0ull};
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.count; t += stride) {
-        uint64_t w = a.base + t;
-        if (w >= *((volatile unsigned long long *)a.found)) return;
+        const uint64_t w = a.base + t;
+        stop.w = w;
+        if (stop()) return;
         uint64_t s[12];
         if (a.ch) {
 #pragma unroll
@@ -264,7 +284,7 @@ __global__ void __launch_bounds__(128) grind_kernel(const __grid_constant__ Grin
             for (uint32_t i = 0; i < a.n_pending; i++) s[i] = a.pending[i];
             s[a.n_pending] = w;
         }
-        p2_permute_dev(s);
+        p2_permute_until(s, stop);  // stopped: the state is noise, but w is above the found one
         if ((p2w::canon(s[7]) & mask) == 0) atomicMin(a.found, (unsigned long long)w);
     }
 }

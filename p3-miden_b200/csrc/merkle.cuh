@@ -185,11 +185,15 @@ __device__ __forceinline__ void ext_linear(uint64_t *s, int rc_off = -1, bool ca
 
 // External rounds take their constants inside the preceding linear layer
 // (rounds 0-3 and 27-29); round 26 follows the internal rounds and adds its own.
-__device__ __forceinline__ void p2_permute_dev(uint64_t *s) {
+// `stop` is asked before each external round and ends the permutation with the
+// state undefined (the proof-of-work search; never for the hashes).
+template <typename Stop>
+__device__ __forceinline__ void p2_permute_until(uint64_t *s, Stop &stop) {
     p2w::ext_linear(s, p2::OFF_INIT);
 #pragma unroll 1
     for (int r = 0; r < 30; r++) {
         if (r < 4 || r >= 26) {
+            if (stop()) return;
             if (r == 26) {
 #pragma unroll
                 for (int i = 0; i < 12; i++) s[i] = p2w::add_c(s[i], c_p2[p2::OFF_TERM + i]);
@@ -210,7 +214,13 @@ __device__ __forceinline__ void p2_permute_dev(uint64_t *s) {
         }
     }
 }
-
+struct NeverStop {
+    __device__ __forceinline__ bool operator()() const { return false; }
+};
+__device__ __forceinline__ void p2_permute_dev(uint64_t *s) {
+    NeverStop stop;
+    p2_permute_until(s, stop);
+}
 
 // Permutation shared by 16 lanes, for latency-bound work (a few states at a
 // time; about 0.28 of the single-thread latency). Lane l < 12 holds word

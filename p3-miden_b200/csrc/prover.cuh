@@ -835,7 +835,7 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
             g.base = base;
             g.count = batch;
             g.found = (unsigned long long *)fb.p;
-            L(fri::grind_kernel, 148 * 2, 128, 0, g);
+            L(fri::grind_kernel, 148 * fri::kGrindBlocks, 128, 0, g);
             ctx.d2h(ctx.stage(1), fb.p, 1);
             ctx.sync();
             found = ctx.pinned[0];
@@ -912,7 +912,7 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
             g.count = 1ull << std::min<uint32_t>(40, fbits + 16);  // ~2^16 times the expected work
             g.found = (unsigned long long *)(dfound.p + r);
             g.ch = devch;
-            L(fri::grind_kernel, 148 * 2, 128, 0, g);
+            L(fri::grind_kernel, 148 * fri::kGrindBlocks, 128, 0, g);
         }
         L(fri::fri_after_grind_kernel, 1, 32, 0, devch, fbits, (const unsigned long long *)(dfound.p + r), dwit.p + r,
           dbeta.p + 2 * r);
