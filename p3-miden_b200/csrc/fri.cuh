@@ -102,43 +102,6 @@ __global__ void __launch_bounds__(128) fold_hash_kernel(const __grid_constant__ 
     }
 }
 
-// The same fold and leaf hash with one 16-lane group per leaf, for rounds
-// with few leaves (latency-bound): lane u < a folds output g*a + u, the leaf
-// words (output i >> 1, component i & 1) are gathered by shuffles, and the
-// group absorbs them (overwrite mode, zero-padded 8-word chunks) with the
-// cooperative permutation.
-__global__ void __launch_bounds__(128) fold_hash_coop_kernel(const __grid_constant__ FoldArgs a) {
-    __shared__ uint64_t sc[p2::N_PARAMS];
-    p2x::stage_consts(sc);
-    const int l = threadIdx.x & 15;
-    const p2x::Lane k = p2x::lane_consts(sc, l);
-    const uint32_t A = 1u << a.log_a;
-    const uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
-    const bool ok = g * A < a.n_out;
-    const uint32_t cnt = ok ? (uint32_t)((a.n_out - g * A) < A ? (a.n_out - g * A) : A) : 0;
-    const gl::ef beta = a.beta_dev ? gl::ef{a.beta_dev[0], a.beta_dev[1]} : a.beta;
-    uint64_t c0 = 0, c1 = 0;
-    if ((uint32_t)l < cnt) {
-        const gl::ef v = fold_any(a, beta, g * A + l);
-        a.out[2 * (g * A + l)] = v.c0;
-        a.out[2 * (g * A + l) + 1] = v.c1;
-        c0 = v.c0, c1 = v.c1;
-    }
-    if (!a.digests) return;  // uniform over the grid
-    const uint32_t W = 2 * A;
-    uint64_t x = 0;
-    for (uint32_t i = 0; i < W; i += 8) {
-        const uint32_t idx = i + (l & 7);
-        const uint64_t w0 = merkle_shfl(c0, (int)(idx >> 1) & 15), w1 = merkle_shfl(c1, (int)(idx >> 1) & 15);
-        if (l < 8) x = idx < W ? ((idx & 1) ? w1 : w0) : 0;
-        x = p2x::permute(x, l, sc, k);
-    }
-    if (cnt == A && l < 4) a.digests[4 * g + l] = p2w::canon(x);
-}
-
-// Proof-of-work search over witnesses [base, base + count): the challenger
-// with `n_pending` buffered inputs observes w and samples; success when the
-// sampled word (state[7] after the duplex) has its low `bits` bits zero.
 // Device copy of the host Challenger (transcript.cuh) for the FRI commit
 // loop: the same observe / sample / duplex rules on canonical words, so the
 // state read back after the loop continues the host transcript unchanged.
@@ -147,11 +110,11 @@ struct DevCh {
     int32_t n_in, n_out;
     int32_t err;  // a grind witness was missing or did not satisfy its bits
 };
-// Warp-cooperative challenger for the one-warp FRI kernels: the DevCh and
-// the constant table are staged in shared memory (WarpChShared), both 16-lane
-// groups of the warp run the duplex permutation (p2x; the second group
-// duplicates the first), group 0 writes the state back and lane 0 does the
-// counters. The observe / sample / duplex rules are the host Challenger's.
+// Warp-cooperative challenger: the DevCh is staged in shared memory beside the
+// constant table (stage_consts, by the whole block), both 16-lane groups of
+// the warp run the duplex permutation (p2x; the second group duplicates the
+// first), group 0 writes the state back and lane 0 does the counters. The
+// observe / sample / duplex rules are the host Challenger's.
 struct WarpChShared {
     DevCh c;
     uint64_t sc[p2::N_PARAMS];
@@ -164,15 +127,8 @@ struct WarpCh {
         const uint32_t *src = (const uint32_t *)g;
         uint32_t *dst = (uint32_t *)&s.c;
         for (uint32_t i = threadIdx.x; i < sizeof(DevCh) / 4; i += 32) dst[i] = src[i];
-        for (int i = threadIdx.x; i < p2::N_PARAMS; i += 32) s.sc[i] = c_p2[i];
         __syncwarp();
         k = p2x::lane_consts(s.sc, l);
-    }
-    __device__ __forceinline__ void store(DevCh *g) {
-        __syncwarp();
-        const uint32_t *src = (const uint32_t *)&s.c;
-        uint32_t *dst = (uint32_t *)g;
-        for (uint32_t i = threadIdx.x; i < sizeof(DevCh) / 4; i += 32) dst[i] = src[i];
     }
     __device__ __forceinline__ void duplex() {
         __syncwarp();
@@ -201,40 +157,105 @@ struct WarpCh {
         return v;
     }
 };
-// send_commit(root): record and observe the four root words (one warp)
-__global__ void __launch_bounds__(32) fri_observe_root_kernel(DevCh *c, const uint64_t *root, uint64_t *log_root) {
-    __shared__ WarpChShared sh;
-    WarpCh w(sh, c);
+// A round of the commit loop between the layer's root and its fold:
+// send_commit(root), grind(bits) with the witness found by grind_kernel, and
+// the folding challenge. What the transcript records is left in the logs.
+struct RoundArgs {
+    const DevCh *ch;  // at the start of the round
+    DevCh *next;      // and at its end: another slot, as every block reads ch
+    const uint64_t *root;
+    uint32_t bits;
+    const unsigned long long *found;
+    uint64_t *log_root, *log_w;
+    uint64_t *beta;
+};
+// By one warp; `writes`: this warp stores the results.
+__device__ __forceinline__ gl::ef round_beta(WarpChShared &sh, const RoundArgs &a, bool writes) {
+    // all loads first: each would wait for memory on its own
+    uint64_t root[4], x = a.bits ? *a.found : 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) root[i] = a.root[i];
+    WarpCh w(sh, a.ch);
+    writes = writes && threadIdx.x == 0;
+#pragma unroll
     for (int i = 0; i < 4; i++) {
-        const uint64_t x = root[i];
-        if (threadIdx.x == 0) log_root[i] = x;
-        w.observe(x);
+        if (writes) a.log_root[i] = root[i];
+        w.observe(root[i]);
     }
-    w.store(c);
-}
-// grind(bits) with the witness found by grind_kernel, then sample the
-// folding challenge beta (one warp)
-__global__ void __launch_bounds__(32) fri_after_grind_kernel(DevCh *c, uint32_t bits, const unsigned long long *found,
-                                                             uint64_t *log_w, uint64_t *beta_out) {
-    __shared__ WarpChShared sh;
-    WarpCh w(sh, c);
-    if (bits == 0) {
-        if (threadIdx.x == 0) *log_w = 0;
+    if (a.bits == 0) {
+        if (writes) *a.log_w = 0;
     } else {
-        uint64_t x = *found;
         if (x == ~0ull) {
             if (threadIdx.x == 0) sh.c.err = 1;
             x = 0;
         }
-        if (threadIdx.x == 0) *log_w = x;
+        if (writes) *a.log_w = x;
         w.observe(x);
-        if ((w.sample() & ((1ull << bits) - 1)) != 0 && threadIdx.x == 0) sh.c.err = 1;
+        if ((w.sample() & ((1ull << a.bits) - 1)) != 0 && threadIdx.x == 0) sh.c.err = 1;
     }
-    const uint64_t b0 = w.sample(), b1 = w.sample();
-    if (threadIdx.x == 0) beta_out[0] = b0, beta_out[1] = b1;
-    w.store(c);
+    gl::ef beta;
+    beta.c0 = w.sample();
+    beta.c1 = w.sample();
+    if (writes) {
+        a.beta[0] = beta.c0, a.beta[1] = beta.c1;
+        *a.next = sh.c;
+    }
+    return beta;
+}
+__global__ void __launch_bounds__(32) fri_round_kernel(const __grid_constant__ RoundArgs a) {
+    __shared__ WarpChShared sh;
+    p2x::stage_consts(sh.sc);
+    round_beta(sh, a, true);
 }
 
+// The same fold and leaf hash with one 16-lane group per leaf, for rounds
+// with few leaves (latency-bound): lane u < a folds output g*a + u, the leaf
+// words (output i >> 1, component i & 1) are gathered by shuffles, and the
+// group absorbs them (overwrite mode, zero-padded 8-word chunks) with the
+// cooperative permutation. Every block's first warp runs the round's challenger
+// itself, which costs no more than a kernel for it would and spares two
+// launches a round (commit phase of 10 / 17 rounds: 1.66 -> 1.55 / 4.62 ->
+// 4.45 ms).
+__global__ void __launch_bounds__(128) fold_hash_coop_kernel(const __grid_constant__ FoldArgs a,
+                                                             const __grid_constant__ RoundArgs r) {
+    __shared__ WarpChShared sh;
+    __shared__ gl::ef beta_sh;
+    const uint64_t *sc = sh.sc;
+    p2x::stage_consts(sh.sc);
+    if (threadIdx.x < 32) {
+        const gl::ef b = round_beta(sh, r, blockIdx.x == 0);
+        if (threadIdx.x == 0) beta_sh = b;
+    }
+    __syncthreads();
+    const gl::ef beta = beta_sh;
+    const int l = threadIdx.x & 15;
+    const p2x::Lane k = p2x::lane_consts(sc, l);
+    const uint32_t A = 1u << a.log_a;
+    const uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+    const bool ok = g * A < a.n_out;
+    const uint32_t cnt = ok ? (uint32_t)((a.n_out - g * A) < A ? (a.n_out - g * A) : A) : 0;
+    uint64_t c0 = 0, c1 = 0;
+    if ((uint32_t)l < cnt) {
+        const gl::ef v = fold_any(a, beta, g * A + l);
+        a.out[2 * (g * A + l)] = v.c0;
+        a.out[2 * (g * A + l) + 1] = v.c1;
+        c0 = v.c0, c1 = v.c1;
+    }
+    if (!a.digests) return;  // uniform over the grid
+    const uint32_t W = 2 * A;
+    uint64_t x = 0;
+    for (uint32_t i = 0; i < W; i += 8) {
+        const uint32_t idx = i + (l & 7);
+        const uint64_t w0 = merkle_shfl(c0, (int)(idx >> 1) & 15), w1 = merkle_shfl(c1, (int)(idx >> 1) & 15);
+        if (l < 8) x = idx < W ? ((idx & 1) ? w1 : w0) : 0;
+        x = p2x::permute(x, l, sc, k);
+    }
+    if (cnt == A && l < 4) a.digests[4 * g + l] = p2w::canon(x);
+}
+
+// Proof-of-work search over witnesses [base, base + count): the challenger
+// with `n_pending` buffered inputs observes w and samples; success when the
+// sampled word (state[7] after the duplex) has its low `bits` bits zero.
 struct GrindArgs {
     uint64_t state[12];
     uint64_t pending[8];
@@ -243,7 +264,8 @@ struct GrindArgs {
     uint64_t base;
     uint64_t count;
     unsigned long long *found;  // atomicMin target, initialised to ~0
-    const DevCh *ch;            // if set, state and pending inputs are read from this device challenger
+    const DevCh *ch;            // if set, the state is read from this device challenger, which has no pending input
+    const uint64_t *root;       // (challenges were sampled last) before the four words of this root
 };
 // A witness below every one this thread could still find is there: the word
 // is asked for a round ahead of its use (it lies in L2).
@@ -274,10 +296,7 @@ __global__ void __launch_bounds__(128) grind_kernel(const __grid_constant__ Grin
         uint64_t s[12];
         if (a.ch) {
 #pragma unroll
-            for (int i = 0; i < 12; i++) s[i] = a.ch->state[i];
-            const int np = a.ch->n_in;
-            for (int i = 0; i < np; i++) s[i] = a.ch->in[i];
-            s[np] = w;
+            for (int i = 0; i < 12; i++) s[i] = i < 4 ? a.root[i] : i == 4 ? w : a.ch->state[i];
         } else {
 #pragma unroll
             for (int i = 0; i < 12; i++) s[i] = a.state[i];

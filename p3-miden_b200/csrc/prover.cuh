@@ -876,9 +876,9 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
         }
     }
     // The rounds run without host round trips: the challenger lives on the
-    // device for the loop (fri::DevCh). Per round: observe the root, grind,
-    // check the witness and sample beta (one-thread kernels), fold + hash the
-    // next round's leaves, compress. The roots, witnesses and the final
+    // device for the loop (fri::DevCh, a slot per round). Per round: grind over
+    // the root's state; observe the root and the witness, sample beta, fold and
+    // hash the next round's leaves; compress. The roots, witnesses and the final
     // challenger state come back in one copy after the loop.
     const uint32_t fbits = pcs.folding_pow_bits;
     const uint64_t n_rounds = rounds;
@@ -889,7 +889,7 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
         memcpy(h.in, tr.ch.in, sizeof(h.in));
         memcpy(h.out, tr.ch.out, sizeof(h.out));
         h.n_in = tr.ch.n_in, h.n_out = tr.ch.n_out, h.err = 0;
-        dch = ctx.alloc((sizeof(fri::DevCh) + 7) / 8);
+        dch = ctx.alloc((n_rounds + 1) * ((sizeof(fri::DevCh) + 7) / 8));
         uint64_t *st = ctx.stage((sizeof(fri::DevCh) + 7) / 8);
         memcpy(st, &h, sizeof(h));
         ctx.h2d(dch.p, st, (sizeof(fri::DevCh) + 7) / 8);
@@ -899,23 +899,24 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
         dfound = ctx.alloc(n_rounds);
         CK(cudaMemsetAsync(dfound.p, 0xff, n_rounds * 8, ctx.stream));
     }
+    static_assert(sizeof(fri::DevCh) % 8 == 0, "slots of whole words");
     fri::DevCh *devch = (fri::DevCh *)dch.p;
     for (uint64_t r = 0; r < n_rounds; r++) {
         Tree &cur = *next_tree;
-        L(fri::fri_observe_root_kernel, 1, 32, 0, devch, (const uint64_t *)(cur.layers.p + 4 * cur.layer_off(cur.depth)),
-          droots.p + 4 * r);
+        const uint64_t *root = cur.layers.p + 4 * cur.layer_off(cur.depth);
+        unsigned long long *found = (unsigned long long *)(dfound.p + r);
         fri_trees.push_back(std::move(next_tree));
         if (fbits) {
             fri::GrindArgs g{};
             g.bits = fbits;
             g.base = 0;
             g.count = 1ull << std::min<uint32_t>(40, fbits + 16);  // ~2^16 times the expected work
-            g.found = (unsigned long long *)(dfound.p + r);
-            g.ch = devch;
+            g.found = found;
+            g.ch = devch + r;
+            g.root = root;
             L(fri::grind_kernel, 148 * fri::kGrindBlocks, 128, 0, g);
         }
-        L(fri::fri_after_grind_kernel, 1, 32, 0, devch, fbits, (const unsigned long long *)(dfound.p + r), dwit.p + r,
-          dbeta.p + 2 * r);
+        const fri::RoundArgs ra{devch + r, devch + r + 1, root, fbits, found, droots.p + 4 * r, dwit.p + r, dbeta.p + 2 * r};
         const uint64_t nout = dom / arity;
         DBuf out = ctx.alloc(2 * nout);
         fri::FoldArgs fa{};
@@ -941,9 +942,11 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
         }
         const uint64_t n_leaves = (nout + arity - 1) / arity;
         if (more && n_leaves <= 4096)  // latency-bound: one 16-lane group per leaf
-            L(fri::fold_hash_coop_kernel, blocks_for(n_leaves * 16, 128), 128, 0, fa);
-        else
+            L(fri::fold_hash_coop_kernel, blocks_for(n_leaves * 16, 128), 128, 0, fa, ra);
+        else {
+            L(fri::fri_round_kernel, 1, 32, 0, ra);
             L(fri::fold_hash_kernel, blocks_for(n_leaves, 128), 128, 0, fa);
+        }
         if (more) {
             compress_layers(ctx, *nt);
             next_tree = std::move(nt);
@@ -956,7 +959,7 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
         ctx.d2h(roots.data(), droots.p, 4 * n_rounds);
         ctx.d2h(wit.data(), dwit.p, n_rounds);
         uint64_t *st = ctx.stage((sizeof(fri::DevCh) + 7) / 8);
-        ctx.d2h(st, dch.p, (sizeof(fri::DevCh) + 7) / 8);
+        ctx.d2h(st, (const uint64_t *)(devch + n_rounds), (sizeof(fri::DevCh) + 7) / 8);
         ctx.sync();
         fri::DevCh h;
         memcpy(&h, st, sizeof(h));
