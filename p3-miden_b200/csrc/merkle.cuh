@@ -637,11 +637,12 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 // The top of a tree, layer l_in up to the root, in one launch of one
-// 8-CTA cluster (4 warps per CTA: one per scheduler, 64 groups): a level's
-// parents are spread over the groups, and the hardware cluster barrier
+// 8-CTA cluster (128 groups; two warps per scheduler at the level of 128
+// parents, which cost 4 us more in two passes of 64 groups): a level's parents
+// are spread over the groups, and the hardware cluster barrier
 // (release / acquire) orders one level's stores before the next level's
 // loads, which read L2 (__ldcg). Warps without a parent in a pass skip it.
-constexpr uint32_t kTopCtas = 8, kTopThreads = 128, kTopGroups = kTopCtas * kTopThreads / 16;
+constexpr uint32_t kTopCtas = 8, kTopThreads = 256, kTopGroups = kTopCtas * kTopThreads / 16;
 __global__ void __cluster_dims__(kTopCtas, 1, 1) __launch_bounds__(kTopThreads)
     compress_top_kernel(uint64_t *layers, uint64_t H, uint32_t l_in, uint32_t depth) {
     __shared__ uint64_t sc[p2::N_PARAMS];
