@@ -19,6 +19,7 @@
 namespace deep {
 
 constexpr int CHUNK = 8;
+constexpr int MAX_DOTS = 24;  // matrices
 
 struct PQArgs {
     uint64_t n;
@@ -78,52 +79,103 @@ __global__ void top_weights_kernel(const uint64_t *q, uint64_t d, uint32_t log_n
 #pragma unroll
     for (int k = 0; k < 4; k++) W[4 * i + k] = gl::mul(q[4 * i + k], x);
 }
-// Wsmall[i] = sum_{c < r} Wbig[i*r + c], eight lanes per i (r is a power of
-// two; a serial sum of 32 was 20 us of load latency)
-__global__ void __launch_bounds__(256) fold_weights_kernel(const uint64_t *Wb, uint64_t n_small, uint64_t r,
-                                                           uint64_t *Ws) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, i = t >> 3;
+// A launch over parts of different sizes: part k has the blocks first[k] <= b <
+// first[k + 1].
+struct Parts {
+    int n = 0;
+    uint32_t first[MAX_DOTS + 1] = {0};
+    void add(uint64_t blocks) { n++, first[n] = first[n - 1] + (uint32_t)blocks; }
+    __device__ __forceinline__ int find(uint32_t &b) const {  // b: the block within its part
+        int k = 0;
+        while (k + 1 < n && first[k + 1] <= b) k++;
+        b -= first[k];
+        return k;
+    }
+};
+
+// W_d of the smaller degrees: Wsmall[i] = sum_{c < r} Wbig[i*r + c], eight
+// lanes per i (r is a power of two; a serial sum of 32 was 20 us of load
+// latency). All degrees in one launch.
+struct FoldWeightsArgs {
+    Parts parts;
+    const uint64_t *Wb;
+    uint64_t n_small[MAX_DOTS], r[MAX_DOTS];
+    uint64_t *Ws[MAX_DOTS];
+};
+__global__ void __launch_bounds__(256) fold_weights_kernel(const __grid_constant__ FoldWeightsArgs a) {
+    uint32_t b = blockIdx.x;
+    const int p = a.parts.find(b);
+    const uint64_t t = (uint64_t)b * blockDim.x + threadIdx.x, i = t >> 3, r = a.r[p];
     const uint32_t lane = threadIdx.x & 7;
     uint64_t s[4] = {0, 0, 0, 0};
-    if (i < n_small)
+    if (i < a.n_small[p])
         for (uint64_t c = lane; c < r; c += 8)
 #pragma unroll
-            for (int k = 0; k < 4; k++) s[k] = gl::add(s[k], Wb[4 * (i * r + c) + k]);
+            for (int k = 0; k < 4; k++) s[k] = gl::add(s[k], a.Wb[4 * (i * r + c) + k]);
 #pragma unroll
     for (int m = 1; m < 8; m <<= 1)
 #pragma unroll
         for (int k = 0; k < 4; k++) s[k] = gl::add(s[k], __shfl_xor_sync(0xffffffffu, s[k], m));
-    if (lane < 4 && i < n_small) Ws[4 * i + lane] = lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3];
+    if (lane < 4 && i < a.n_small[p]) a.Ws[p][4 * i + lane] = lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3];
 }
 
-// Column sums: partial[chunk][col][0..4) = sum over rows of chunk of
-// W[i][j] * M[i][col] (EF for j = 0, 1). Block: 32 columns x 8 row lanes.
-__global__ void __launch_bounds__(256) colsum_kernel(const uint64_t *M, uint64_t w, uint64_t d, const uint64_t *W,
-                                                     uint64_t rows_per_chunk, uint64_t *partial) {
+// Column sums of all matrices: partial[chunk][col][0..4) = sum over the
+// chunk's rows of W[i][j] * M[i][col] (EF for j = 0, 1). A block takes 32
+// columns x 8 row lanes of one chunk; all chunks have the same number of rows,
+// so that the blocks of all matrices, one wave, end together. Four rows per
+// step, loaded a step ahead; the weights of kTileRows rows in shared memory,
+// a tile ahead. Bound by the integer pipes and latency (floors at 2^17 x 2633
+// words: 0.42 ms of memory, 0.62 of products): the opening call over one such
+// matrix takes 1.17 ms; 1.26 with both loads waited for in each step, 1.45
+// with only the words ahead, 1.31 with eight rows per step (two blocks per
+// SM), 1.58 at 64 registers (four).
+struct ColsumArgs {
+    Parts parts;
+    const uint64_t *M[MAX_DOTS], *W[MAX_DOTS];
+    uint64_t w[MAX_DOTS], d[MAX_DOTS];
+    uint64_t *partial[MAX_DOTS];
+    uint64_t rows_per_chunk;
+};
+constexpr int kTileRows = 128;
+__global__ void __launch_bounds__(256) colsum_kernel(const __grid_constant__ ColsumArgs a) {
     __shared__ uint64_t red[8][32][4];
+    __shared__ ulonglong2 wt[2][2 * kTileRows];
+    uint32_t b = blockIdx.x;
+    const int p = a.parts.find(b);
+    const uint64_t w = a.w[p];
+    const uint32_t tiles = (uint32_t)((w + 31) / 32), chunk = b / tiles;
     const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
-    // grid: x = column tile (fastest), y = row chunk
-    const uint64_t col = (uint64_t)blockIdx.x * 32 + cl;
-    const uint64_t r0 = (uint64_t)blockIdx.y * rows_per_chunk;
-    const uint64_t r1 = min(d, r0 + rows_per_chunk);
+    const uint64_t col = (uint64_t)(b - chunk * tiles) * 32 + cl;
+    const uint64_t r0 = chunk * a.rows_per_chunk, r1 = min(a.d[p], r0 + a.rows_per_chunk);
+    const uint64_t *M = a.M[p] + col;
+    const ulonglong2 *W = (const ulonglong2 *)a.W[p];
+    // a tile of kTileRows weights: half a row (16 bytes) per thread
+    auto weights = [&](uint64_t tile) {
+        const uint64_t e = 2 * tile + threadIdx.x;
+        return e < 2 * r1 ? __ldg(W + e) : ulonglong2{0, 0};
+    };
+    auto word = [&](uint64_t i) { return col < w && i < r1 ? __ldg(M + i * w) : 0; };
     gl::SplitAcc acc[4];
-    if (col < w) {
-        // four rows per step: their loads are issued together, so that each
-        // thread keeps several DRAM reads in flight
-        uint64_t i = r0 + rl;
-        for (; i + 24 < r1; i += 32) {
-            uint64_t v[4];
+    uint64_t v[4], nv[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = __ldg(M + (i + 8 * u) * w + col);
+    for (int u = 0; u < 4; u++) v[u] = word(r0 + rl + 8 * u);
+    ulonglong2 nw = weights(r0);
+    for (uint64_t tile = r0; tile < r1; tile += kTileRows) {
+        const int buf = (int)((tile - r0) / kTileRows) & 1;
+        wt[buf][threadIdx.x] = nw;
+        __syncthreads();  // also: the tile before last is read
+        nw = weights(tile + kTileRows);
 #pragma unroll
-            for (int u = 0; u < 4; u++)
+        for (int q = 0; q < kTileRows; q += 32) {
 #pragma unroll
-                for (int k = 0; k < 4; k++) acc[k].mac(v[u], __ldg(W + 4 * (i + 8 * u) + k));
-        }
-        for (; i < r1; i += 8) {
-            uint64_t v = __ldg(M + i * w + col);
+            for (int u = 0; u < 4; u++) nv[u] = word(tile + q + 32 + rl + 8 * u);
 #pragma unroll
-            for (int k = 0; k < 4; k++) acc[k].mac(v, __ldg(W + 4 * i + k));
+            for (int u = 0; u < 4; u++) {
+                const ulonglong2 w0 = wt[buf][2 * (q + rl + 8 * u)], w1 = wt[buf][2 * (q + rl + 8 * u) + 1];
+                acc[0].mac(v[u], w0.x), acc[1].mac(v[u], w0.y), acc[2].mac(v[u], w1.x), acc[3].mac(v[u], w1.y);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = nv[u];
         }
     }
     uint64_t s[4];
@@ -135,17 +187,26 @@ __global__ void __launch_bounds__(256) colsum_kernel(const uint64_t *M, uint64_t
 #pragma unroll
             for (int k = 0; k < 4; k++) s[k] = gl::add(s[k], red[r][cl][k]);
 #pragma unroll
-        for (int k = 0; k < 4; k++) partial[(blockIdx.y * w + col) * 4 + k] = s[k];
+        for (int k = 0; k < 4; k++) a.partial[p][(chunk * w + col) * 4 + k] = s[k];
     }
 }
 // out[col][0..4) = s_j * sum_chunk partial[chunk][col]: a block sums 8 columns
 // (32 words, contiguous in a chunk) with 16 rows of threads over the chunks;
 // with one thread per column, 296 chunks of a narrow matrix took 157 us.
-__global__ void __launch_bounds__(512) colsum_finish_kernel(const uint64_t *partial, uint64_t n_chunks, uint64_t w,
-                                                            gl::ef s0, gl::ef s1, uint64_t *out) {
+struct ColsumFinishArgs {
+    Parts parts;
+    const uint64_t *partial[MAX_DOTS];
+    uint64_t n_chunks[MAX_DOTS], w[MAX_DOTS];
+    uint64_t *out[MAX_DOTS];
+    gl::ef s0, s1;
+};
+__global__ void __launch_bounds__(512) colsum_finish_kernel(const __grid_constant__ ColsumFinishArgs a) {
     __shared__ uint64_t red[16][32];
+    uint32_t b = blockIdx.x;
+    const int p = a.parts.find(b);
+    const uint64_t w = a.w[p], n_chunks = a.n_chunks[p], *partial = a.partial[p];
     const uint32_t e = threadIdx.x & 31, r = threadIdx.x >> 5;
-    const uint64_t word = (uint64_t)blockIdx.x * 32 + e;
+    const uint64_t word = (uint64_t)b * 32 + e;
     uint64_t s = 0;
     if (word < 4 * w)
 #pragma unroll 4
@@ -158,23 +219,24 @@ __global__ void __launch_bounds__(512) colsum_finish_kernel(const uint64_t *part
     // the four words of a column are four neighbouring lanes
     const uint64_t c1 = __shfl_down_sync(0xffffffffu, s, 1);
     if (word < 4 * w && !(e & 1)) {
-        const gl::ef v = gl::ef_mul(gl::ef{s, c1}, (e & 2) ? s1 : s0);
-        out[word] = v.c0;
-        out[word + 1] = v.c1;
+        const gl::ef v = gl::ef_mul(gl::ef{s, c1}, (e & 2) ? a.s1 : a.s0);
+        a.out[p][word] = v.c0;
+        a.out[p][word + 1] = v.c1;
     }
 }
 
 // The column coefficients -ac^{W-1-c} over the aligned columns of all
 // matrices, and the reduced openings f_red(z_j) = sum_c ac^{W-1-c} f_c(z_j)
 // (padding columns are zero). One block: ac^0..ac^1023 by doubling in shared
-// memory, then 1024 columns at a time from the last (at 1338 columns 22 us cold,
-// 33 with a power per column; on the host it was an upload and two waits).
-constexpr int MAX_DOTS = 24;
+// memory with the powers ac^(2^s) from the host (squared in every thread they
+// were half of the block's products), then 1024 columns at a time from the
+// last (at 1338 columns 12 us cold, 22 with the squarings; on the host it was
+// an upload and two waits).
 struct CoefArgs {
     int n_mats;
     uint64_t w[MAX_DOTS], off[MAX_DOTS], aligned_off[MAX_DOTS];  // columns and their places in evals and coef
     uint64_t total_aligned;
-    gl::ef ac;
+    gl::ef step[11];  // ac^(2^s)
     const uint64_t *evals;  // 4 words per column: f(z_0), f(z_1)
     uint64_t *coef;         // 2 words per aligned column; the padding's are not written
     uint64_t *fred;         // 4 words
@@ -184,11 +246,10 @@ __global__ void __launch_bounds__(1024) coef_kernel(const __grid_constant__ Coef
     __shared__ uint64_t red[32][4];
     const uint32_t tid = threadIdx.x;
     if (tid == 0) pw[0] = gl::ef_one();
-    gl::ef step = a.ac;  // ac^(2^s)
-    for (uint32_t n = 1; n < 1024; n *= 2) {
+#pragma unroll 1
+    for (int s = 0; s < 10; s++) {
         __syncthreads();
-        if (tid >= n && tid < 2 * n) pw[tid] = gl::ef_mul(pw[tid - n], step);
-        step = gl::ef_sqr(step);
+        if (tid >> s == 1) pw[tid] = gl::ef_mul(pw[tid - (1u << s)], a.step[s]);
     }
     __syncthreads();
     gl::ef p = pw[tid], f[2] = {gl::ef_zero(), gl::ef_zero()};
@@ -205,7 +266,7 @@ __global__ void __launch_bounds__(1024) coef_kernel(const __grid_constant__ Coef
             f[0] = gl::ef_add(f[0], gl::ef_mul(p, gl::ef{v[0], v[1]}));
             f[1] = gl::ef_add(f[1], gl::ef_mul(p, gl::ef{v[2], v[3]}));
         }
-        p = gl::ef_mul(p, step);  // ac^1024
+        p = gl::ef_mul(p, a.step[10]);
     }
     uint64_t s[4] = {f[0].c0, f[0].c1, f[1].c0, f[1].c1};
 #pragma unroll
@@ -227,7 +288,9 @@ __global__ void __launch_bounds__(1024) coef_kernel(const __grid_constant__ Coef
 // per row (about eight columns per lane at least, so that the reduction over
 // the lanes does not count: 2^18 x 64 took 111 us with 32 lanes per row, 47
 // with 8; 2^16 x 250 74 us with 32, 42 with 16), coefficients staged in shared
-// memory. Bound by the integer pipes (two lazy products per word).
+// memory. Bound by memory at large widths and the integer pipes (two lazy
+// products per word): the quotient call over 2^18 x 2633 words takes 1.11 ms,
+// 1.23 with the loads of a step waited for.
 template <int G>
 __global__ void __launch_bounds__(256) rowdot_lanes_kernel(const uint64_t *M, uint64_t h, uint64_t w,
                                                            const uint64_t *coef, uint64_t *dots) {
@@ -238,22 +301,35 @@ __global__ void __launch_bounds__(256) rowdot_lanes_kernel(const uint64_t *M, ui
     const uint32_t lane = threadIdx.x % G;
     const uint64_t rows = (uint64_t)gridDim.x * (blockDim.x / G);
     const uint64_t first = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-    // every lane of a warp takes the same number of turns
-    for (uint64_t base = first - (threadIdx.x % 32) / G; base < h; base += rows) {
-        const uint64_t i = base + (threadIdx.x % 32) / G;
-        const uint64_t *row = M + (i < h ? i : h - 1) * w;
-        gl::SplitAcc a0, a1;
-        for (uint64_t col = lane; col < padded; col += 4 * G) {  // four loads in flight per lane
-            uint64_t v[4];
+    // every lane of a warp takes the same number of turns; a step's words are
+    // loaded during the step before, the next row's first ones included
+    const uint32_t sub = (threadIdx.x % 32) / G;
+    auto row_at = [&](uint64_t i) { return M + (i < h ? i : h - 1) * w; };
+    const uint64_t *row = row_at(first);
+    uint64_t v[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = col + G * u < w ? __ldg(row + col + G * u) : 0;
+    for (int u = 0; u < 4; u++) v[u] = lane + G * u < w ? __ldg(row + lane + G * u) : 0;
+    for (uint64_t base = first - sub; base < h; base += rows) {
+        const uint64_t i = base + sub;
+        const uint64_t *next_row = row_at(i + rows);
+        gl::SplitAcc a0, a1;
+        for (uint64_t col = lane; col < padded; col += 4 * G) {
+            const bool more = col + 4 * G < padded;
+            const uint64_t *from = more ? row : next_row;
+            const uint64_t c = more ? col + 4 * G : lane;
+            uint64_t nv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) nv[u] = c + G * u < w ? __ldg(from + c + G * u) : 0;
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const ulonglong2 k = *(const ulonglong2 *)(sc + 2 * (col + G * u));
                 a0.mac(v[u], k.x);
                 a1.mac(v[u], k.y);
             }
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = nv[u];
         }
+        row = next_row;
         uint64_t c0 = a0.reduce(), c1 = a1.reduce();
 #pragma unroll
         for (int off = G / 2; off; off >>= 1) {

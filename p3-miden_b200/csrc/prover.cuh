@@ -479,11 +479,17 @@ inline std::vector<uint64_t> deep_evals(Ctx &ctx, Launcher &L, const std::vector
     weights[d] = ctx.alloc(4 * d);
     L(deep::top_weights_kernel, blocks_for(d, 256), 256, 0, st.q.p, d, log_lde,
       ntt::PowTab{twn.fwd_lo.p, twn.fwd_hi.p, twn.lo_bits}, weights[d].p);
-    for (const Mat *m : all) {
-        uint64_t dm = m->h >> lb;
-        if (weights.count(dm)) continue;
-        weights[dm] = ctx.alloc(4 * dm);
-        L(deep::fold_weights_kernel, blocks_for(dm * 8, 256), 256, 0, weights[d].p, dm, d / dm, weights[dm].p);
+    {
+        deep::FoldWeightsArgs fa{};
+        for (const Mat *m : all) {
+            const uint64_t dm = m->h >> lb;
+            if (weights.count(dm)) continue;
+            weights[dm] = ctx.alloc(4 * dm);
+            fa.n_small[fa.parts.n] = dm, fa.r[fa.parts.n] = d / dm, fa.Ws[fa.parts.n] = weights[dm].p;
+            fa.parts.add(blocks_for(dm * 8, 256));
+        }
+        fa.Wb = weights[d].p;
+        if (fa.parts.n) L(deep::fold_weights_kernel, fa.parts.first[fa.parts.n], 256, 0, fa);
     }
     gl::ef sj[2];
     for (int j = 0; j < 2; j++) {
@@ -494,27 +500,39 @@ inline std::vector<uint64_t> deep_evals(Ctx &ctx, Launcher &L, const std::vector
     st.evals = ctx.alloc(4 * total_w);
     DBuf &evals = st.evals;
     {
-        uint64_t off = 0;
-        for (const Mat *m : all) {
-            uint64_t dm = m->h >> lb;
-            uint64_t col_tiles = (m->w + 31) / 32;
-            // one wave of resident blocks: as many row chunks as fit beside the
-            // column tiles (a second, partial wave would double the time)
-            int bps = 0, sms = 0;
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, deep::colsum_kernel, 256, 0));
-            CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
-            bps = std::max(1, bps);
-            const uint64_t target_blocks = (uint64_t)sms * bps;
-            uint64_t n_chunks = std::max<uint64_t>(1, std::min<uint64_t>(dm / 64 + 1, target_blocks / col_tiles));
-            uint64_t rpc = (dm + n_chunks - 1) / n_chunks;
-            n_chunks = (dm + rpc - 1) / rpc;
-            DBuf part = ctx.alloc(n_chunks * m->w * 4);
-            L(deep::colsum_kernel, dim3((unsigned)col_tiles, (unsigned)n_chunks), 256, 0, m->d, m->w, dm,
-              weights[dm].p, rpc, part.p);
-            L(deep::colsum_finish_kernel, blocks_for(m->w * 4, 32), 512, 0, part.p, n_chunks, m->w, sj[0], sj[1],
-              evals.p + 4 * off);
-            off += m->w;
+        // one wave of resident blocks over all matrices: the fewest rows per
+        // chunk that fit (a second, partial wave would double the time)
+        int bps = 0, sms = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, deep::colsum_kernel, 256, 0));
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+        const uint64_t target_blocks = (uint64_t)sms * std::max(1, bps);
+        auto blocks = [&](uint64_t rows) {
+            uint64_t b = 0;
+            for (const Mat *m : all) b += (m->w + 31) / 32 * (((m->h >> lb) + rows - 1) / rows);
+            return b;
+        };
+        uint64_t rows = 64;
+        while (rows < d && blocks(rows) > target_blocks) rows += (rows + 31) / 32;
+        deep::ColsumArgs ca{};
+        deep::ColsumFinishArgs fa{};
+        ca.rows_per_chunk = rows;
+        fa.s0 = sj[0], fa.s1 = sj[1];
+        uint64_t words = 0, off = 0;
+        for (const Mat *m : all) words += ((m->h >> lb) + rows - 1) / rows * m->w * 4;
+        DBuf part = ctx.alloc(words);
+        words = 0;
+        for (size_t mi = 0; mi < all.size(); mi++) {
+            const Mat *m = all[mi];
+            const uint64_t dm = m->h >> lb, n_chunks = (dm + rows - 1) / rows;
+            ca.M[mi] = m->d, ca.W[mi] = weights[dm].p, ca.w[mi] = fa.w[mi] = m->w, ca.d[mi] = dm;
+            ca.partial[mi] = part.p + words, fa.partial[mi] = part.p + words;
+            fa.n_chunks[mi] = n_chunks, fa.out[mi] = evals.p + 4 * off;
+            ca.parts.add((m->w + 31) / 32 * n_chunks);
+            fa.parts.add(blocks_for(m->w * 4, 32));
+            words += n_chunks * m->w * 4, off += m->w;
         }
+        L(deep::colsum_kernel, ca.parts.first[all.size()], 256, 0, ca);
+        L(deep::colsum_finish_kernel, fa.parts.first[all.size()], 512, 0, fa);
     }
     std::vector<uint64_t> h_evals(4 * total_w);
     ctx.d2h(h_evals.data(), evals.p, 4 * total_w);
@@ -551,7 +569,8 @@ inline DBuf deep_assemble(Ctx &ctx, Launcher &L, const std::vector<const Mat *> 
             off += all[mi]->w, aoff += st.aligned_w[mi];
         }
         c.total_aligned = total_aligned;
-        c.ac = ac;
+        c.step[0] = ac;
+        for (int k = 1; k < 11; k++) c.step[k] = gl::ef_sqr(c.step[k - 1]);
         c.evals = st.evals.p;
         c.coef = d_coef.p;
         c.fred = d_fred.p;
