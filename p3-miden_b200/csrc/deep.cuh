@@ -64,9 +64,7 @@ __global__ void __launch_bounds__(128) point_quotients_kernel(const __grid_const
             const int e = 2 * t + j;
             const uint64_t ni = gl::mul(inv, pre[e]);
             inv = gl::mul(inv, norm[e]);
-            uint64_t *o = a.q + 4 * (i0 + t) + 2 * j;
-            o[0] = gl::mul(d[e], ni);
-            o[1] = gl::mul(gl::neg(a.z[j].c1), ni);
+            ((ulonglong2 *)a.q)[2 * (i0 + t) + j] = ulonglong2{gl::mul(d[e], ni), gl::mul(gl::neg(a.z[j].c1), ni)};
         }
     }
 }
@@ -285,10 +283,11 @@ __global__ void __launch_bounds__(1024) coef_kernel(const __grid_constant__ Coef
 }
 
 // Row dot products dots[i] = sum_col coef[col] * M[i][col] (EF coef), G lanes
-// per row (about eight columns per lane at least, so that the reduction over
-// the lanes does not count: 2^18 x 64 took 111 us with 32 lanes per row, 47
-// with 8; 2^16 x 250 74 us with 32, 42 with 16), coefficients staged in shared
-// memory. Bound by memory at large widths and the integer pipes (two lazy
+// per row: about 32 columns per lane at least, as the reduction over the lanes
+// costs as much as the products of eleven columns (the quotient call over
+// 2^18 x 64 / 2^17 x 128 / 2^16 x 256 / 2^16 x 512 / 2^15 x 800 takes 133 / 131
+// / 128 / 149 / 139 us, with twice as many lanes 141 / 132 / 131 / 158 / 146).
+// Coefficients staged in shared memory. Bound by memory at large widths and the integer pipes (two lazy
 // products per word): the quotient call over 2^18 x 2633 words takes 1.11 ms,
 // 1.23 with the loads of a step waited for.
 template <int G>

@@ -584,9 +584,9 @@ inline DBuf deep_assemble(Ctx &ctx, Launcher &L, const std::vector<const Mat *> 
             const Mat *m = all[mi];
             dots[mi] = ctx.alloc(2 * m->h);
             const uint64_t *cf = d_coef.p + 2 * off;
-            if (m->w >= 256) launch_rowdot<32>(L, m, cf, dots[mi].p);
-            else if (m->w >= 128) launch_rowdot<16>(L, m, cf, dots[mi].p);
-            else if (m->w >= 64) launch_rowdot<8>(L, m, cf, dots[mi].p);
+            if (m->w >= 1024) launch_rowdot<32>(L, m, cf, dots[mi].p);
+            else if (m->w >= 512) launch_rowdot<16>(L, m, cf, dots[mi].p);
+            else if (m->w >= 256) launch_rowdot<8>(L, m, cf, dots[mi].p);
             else if (m->w >= 16) launch_rowdot<4>(L, m, cf, dots[mi].p);
             else L(deep::rowdot_thread_kernel, blocks_for(m->h, 256), 256, 0, m->d, m->h, m->w, cf, dots[mi].p);
             aa.dots[mi] = dots[mi].p;
