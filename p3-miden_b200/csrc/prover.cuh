@@ -218,19 +218,24 @@ inline void commit_main_pipelined(Ctx &ctx, const Instance *inst, size_t n_inst,
     for (size_t i = 0; i < n_inst; i++) {
         uint64_t w = inst[i].width, h = inst[i].height;
         if (!inst[i].trace_on_device && w >= 256) {
-            // a wide host trace: slabs that grow geometrically (x1.5, multiples of
-            // the rate 8) from about 1/64 of the width, so that only the small
-            // first slab's upload is exposed and each later upload (PCIe) fits
-            // under the LDE and hash of the slab before it (about 1.6x the
-            // upload time per column on a B200 at blowup 2, more at larger
-            // blowups)
+            // a wide host trace: slabs that grow geometrically (multiples of the
+            // rate 8) from about 1/64 of the width, so that only the small first
+            // slab's upload is exposed and each later upload (PCIe) fits under
+            // the LDE and hash of the slab before it: about 1.23x the upload time
+            // per column at blowup 2 (47 against 38 us at 2^18 rows), more at
+            // larger blowups, hence x1.2 (2^18 x 2633: a proof from a host trace
+            // takes 157 ms, 160 at x1.25, 172 at x1.5, against 151 from a
+            // resident one). Below 2^14 rows the upload is short and a launch
+            // counts for more: x1.5 (2^12 / 2^14 rows: 11.2 / 20.8 ms, at x1.2
+            // 11.4 / 20.4).
+            const uint64_t num = h >= 1 << 14 ? 6 : 3, den = h >= 1 << 14 ? 5 : 2;
             uint64_t cur = std::max<uint64_t>(8, (w / 64 + 7) / 8 * 8);
             for (uint64_t c0 = 0; c0 < w;) {
                 const uint64_t take = std::min(cur, w - c0);
                 slabs.push_back({i, c0, take});
                 max_slab_hw = std::max(max_slab_hw, h * take);
                 c0 += take;
-                cur = (cur * 3 / 2 + 7) / 8 * 8;
+                cur = (cur * num / den + 7) / 8 * 8;
             }
         } else {
             uint64_t sw = w >= 256 ? ((w + 7) / 8 + 7) / 8 * 8 : w;  // about 8 slabs for wide traces
