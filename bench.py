@@ -276,12 +276,13 @@ def slab_widths(w: int):
 
 def hash_roofline(n_lde: int, w: int, leaf_ms: float, n_launches: int, hbm_peak: float, peak_src: str,
                   sm_mhz, profile: Path = HASH_PROFILE):
-    """Roofline line of the dominant kernel, merkle::leaf_class_kernel (one
-    launch per column slab). It is bound by the integer ALU pipe: achieved =
-    this run's ALU-pipe warp instructions per second (the live launch time
-    times the per-permutation ALU count of the committed ncu summary), peak =
-    the pipe's rate at this run's SM clock (from the same summary's
-    instruction count and % of peak). The HBM figures sit beside it."""
+    """Roofline line of the dominant kernel, merkle::leaf_class_tc_kernel (one
+    launch per column slab). It is bound by the integer multiplier pipe, with
+    the ALU pipe close behind: achieved = this run's warp instructions per
+    second on that pipe (the live launch time times the per-permutation count
+    of the committed ncu summary), peak = the pipe's rate at this run's SM
+    clock (from the same summary's instruction count and % of peak). The ALU
+    pipe's and the HBM figures sit beside it."""
     n_launches = max(1, n_launches)
     launch_s = leaf_ms / 1e3 / n_launches
     perms = n_lde * sum((x + 7) // 8 for x in slab_widths(w))
@@ -290,26 +291,33 @@ def hash_roofline(n_lde: int, w: int, leaf_ms: float, n_launches: int, hbm_peak:
     hbm_gbs = alg_bytes / launch_s / 1e9
     hbm = {"achieved": hbm_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": hbm_gbs / hbm_peak,
            "peak_source": peak_src, "algorithmic_bytes": alg_bytes}
-    base = {"kernel": "merkle::leaf_class_kernel (LMCS leaf sponge, Poseidon2-12)", "kernel_ms": launch_s * 1e3,
+    base = {"kernel": "merkle::leaf_class_tc_kernel (LMCS leaf sponge, Poseidon2-12)", "kernel_ms": launch_s * 1e3,
             "launches_per_proof": n_launches, "perms_per_launch": perms_per_launch,
             "perms_per_s": perms_per_launch / launch_s, "algorithmic_bytes": alg_bytes}
     prof = load_profile(profile)
     if not prof:
         return {**base, "bound": "hbm", "achieved": hbm_gbs, "peak": hbm_peak, "unit": "GB/s",
                 "frac": hbm_gbs / hbm_peak, "traffic": None, "peak_source": peak_src}
-    alu_per_perm = prof["inst_alu"] / prof["perms_per_launch"]
-    # the pipe's peak rate from the full-size slab capture (a small capture
+    # the pipes' peak rates from the full-size slab capture (a small capture
     # leaves SMs idle in its tail, which understates the rate)
     pk = load_profile(HASH_PROFILE) or prof
-    peak_rate = pk["inst_alu"] / (pk["duration_ns"] * 1e-9) / (pk["alu_pct_of_peak"] / 100.0)
-    if sm_mhz and pk.get("sm_mhz"):
-        peak_rate *= sm_mhz / pk["sm_mhz"]
-    achieved = perms_per_launch * alu_per_perm / launch_s
-    return {**base, "bound": "int_alu", "achieved": achieved / 1e9, "peak": peak_rate / 1e9,
-            "unit": "G warp-instructions/s (ALU pipe)", "frac": achieved / peak_rate,
+
+    def pipe(inst: str, pct: str):
+        per_perm = prof[inst] / prof["perms_per_launch"]
+        peak = pk[inst] / (pk["duration_ns"] * 1e-9) / (pk[pct] / 100.0)
+        if sm_mhz and pk.get("sm_mhz"):
+            peak *= sm_mhz / pk["sm_mhz"]
+        return per_perm, perms_per_launch * per_perm / launch_s, peak
+
+    mul_per_perm, achieved, peak_rate = pipe("inst_fmaheavy", "fmaheavy_pct_of_peak")
+    alu_per_perm, alu_achieved, alu_peak = pipe("inst_alu", "alu_pct_of_peak")
+    return {**base, "bound": "int_mul", "achieved": achieved / 1e9, "peak": peak_rate / 1e9,
+            "unit": "G warp-instructions/s (multiplier pipe)", "frac": achieved / peak_rate,
             "traffic": prof["dram_bytes"] / prof["perms_per_launch"] * perms_per_launch,
-            "alu_inst_per_perm": alu_per_perm, "issue_frac_in_profile": prof["issue_pct"] / 100.0,
-            "peak_source": f"ALU-pipe rate from {HASH_PROFILE.relative_to(ROOT)}; instructions per permutation "
+            "mul_inst_per_perm": mul_per_perm, "issue_frac_in_profile": prof["issue_pct"] / 100.0,
+            "alu_pipe": {"achieved": alu_achieved / 1e9, "peak": alu_peak / 1e9, "frac": alu_achieved / alu_peak,
+                         "inst_per_perm": alu_per_perm},
+            "peak_source": f"pipe rates from {HASH_PROFILE.relative_to(ROOT)}; instructions per permutation "
                            f"and DRAM traffic from {profile.relative_to(ROOT)}", "hbm": hbm}
 
 
@@ -319,7 +327,7 @@ def lde_roofline(w: int, B: int, lde_ms: float, hbm_peak: float, sm_mhz):
     ALU pipe, scaled from the committed ncu summary by algorithmic bytes."""
     lde_bytes = 8.0 * w * (1 << LOG_H) * (1 + B)
     gbs = lde_bytes / (lde_ms * 1e-3) / 1e9
-    out = {"kernel": "lde::lde_pass_kernel + lde::lde_fused_kernel (coset LDE, 3 launches x 8 slabs)",
+    out = {"kernel": "lde::lde_pass_tile_kernel + lde::lde_fused_tile_kernel (coset LDE, 3 launches per column slab)",
            "bound": "hbm", "achieved": gbs, "peak": hbm_peak, "unit": "GB/s", "frac": gbs / hbm_peak,
            "algorithmic_bytes": lde_bytes, "kernel_ms": lde_ms, "traffic": None}
     prof = load_profile(LDE_PROFILE)
@@ -454,7 +462,7 @@ def run_gpu(args):
                              "measured" if "hbm_gbs" in pk else "fallback", clk.get("sm_mhz"),
                              HASH_PROFILE_CM if cm else HASH_PROFILE)
     if cm:
-        roofline["kernel"] = ("merkle::leaf_class_kernel<true> (LMCS leaf sponge, Poseidon2-12; also writes "
+        roofline["kernel"] = ("merkle::leaf_class_tc_kernel<true> (LMCS leaf sponge, Poseidon2-12; also writes "
                               "the column-major rows the generated constraint kernels read)")
     lde = lde_roofline(w, B, float(np.mean(lde_k)), hbm_peak, clk.get("sm_mhz"))
     line = {
