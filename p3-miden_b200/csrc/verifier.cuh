@@ -100,9 +100,34 @@ __global__ void __launch_bounds__(128) leaf_kernel(const LeafJob *jobs, uint32_t
     if (threadIdx.x % 32 < 4) pool[4 * (uint64_t)job.out + l] = p2w::canon(x);
 }
 
-// The same sponge with one thread per leaf, for large batches: with many
-// leaves in flight throughput decides, and the single-thread permutation
-// costs about a fifth of the cooperative one's issue slots.
+// The same sponge with four lanes per leaf, for batches: the longest rows of a
+// batch (330 chained permutations for the Keccak trace) are a small part of its
+// leaves, and their chain decides. The eight leaves of a warp permute together;
+// one that has ended keeps its state.
+__global__ void __launch_bounds__(128) leaf_quad_kernel(const LeafJob *jobs, uint32_t n, const uint64_t *rows,
+                                                        const uint32_t *widths, uint64_t *pool) {
+    __shared__ uint64_t sc[p2::N_PARAMS];
+    p2x::stage_consts(sc);
+    const int l = threadIdx.x & 3;
+    const p2q::Lane k = p2q::lane_consts(sc, l);
+    const uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const LeafJob job = j < n ? jobs[j] : LeafJob{};  // past the end: no matrix
+    const uint64_t *row = rows + job.row_off;
+    uint64_t x[3] = {0, 0, 0};
+    for (uint32_t m = 0, i = 0, w = 0;; i += 8) {
+        while (i >= w && m < job.n_w) row += w, w = widths[job.w_off + m++], i = 0;
+        const bool more = i < w;
+        if (!__any_sync(0xffffffffu, more)) break;
+        uint64_t y[3] = {x[0], x[1], x[2]};
+        if (more) y[0] = i + l < w ? row[i + l] : 0, y[1] = i + 4 + l < w ? row[i + 4 + l] : 0;
+        p2q::permute(y, sc, k);
+        if (more) x[0] = y[0], x[1] = y[1], x[2] = y[2];
+    }
+    if (j < n) pool[4 * (uint64_t)job.out + l] = p2w::canon(x[0]);
+}
+
+// The same sponge with one thread per leaf, for the largest batches: with that
+// many leaves in flight throughput decides.
 __global__ void __launch_bounds__(128) leaf_thread_kernel(const LeafJob *jobs, uint32_t n, const uint64_t *rows,
                                                           const uint32_t *widths, uint64_t *pool) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -120,7 +145,11 @@ __global__ void __launch_bounds__(128) leaf_thread_kernel(const LeafJob *jobs, u
 #pragma unroll
     for (int i = 0; i < 4; i++) pool[4 * (uint64_t)job.out + i] = p2w::canon(s[i]);
 }
-constexpr uint32_t kThreadLeaves = 2048;  // from this many leaves on, one thread per leaf
+// Four lanes per leaf from kQuadLeaves leaves on, one thread from kThreadLeaves
+// on. 4 / 8 / 16 / 32 / 64 proofs of 2^18 Keccak rows (about 2100 leaves each):
+// device part of the call 3.8 / 4.4 / 6.5 / 9.0 / 14.0 ms with four lanes, 8.8 /
+// 9.4 / 13.6 / 14.6 / 16.6 with one thread; the lines meet at about 90 proofs.
+constexpr uint32_t kQuadLeaves = 2048, kThreadLeaves = 3u << 16;
 
 // The compressions of one tree level of every proof: 16 lanes each (p2x), or
 // four (p2q), or one thread, by how many there are (launch_compress).
@@ -894,6 +923,9 @@ inline void device_pass(Ctx &ctx, const std::vector<Prepared *> &vs, Timing *tm,
             leaf_thread_kernel<<<(n + 127) / 128, 128, 0, ctx.stream>>>((const LeafJob *)(d.p + o_leaves), n,
                                                                         d.p + o_rows, (const uint32_t *)(d.p + o_widths),
                                                                         pool);
+        else if (n >= kQuadLeaves)
+            leaf_quad_kernel<<<(n * 4 + 127) / 128, 128, 0, ctx.stream>>>((const LeafJob *)(d.p + o_leaves), n, d.p + o_rows,
+                                                                          (const uint32_t *)(d.p + o_widths), pool);
         else
             leaf_kernel<<<(n * 32 + 127) / 128, 128, 0, ctx.stream>>>((const LeafJob *)(d.p + o_leaves), n,
                                                                       d.p + o_rows, (const uint32_t *)(d.p + o_widths),

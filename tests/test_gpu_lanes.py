@@ -34,9 +34,9 @@ def test_deep_of_every_width(product, gpu_ctx, widths, alignment, kind):
     assert np.array_equal(q, O.deep_quotient(mats, lb, alignment, zs, ev, alpha, beta))
 
 
-# about 400 leaves and as many compressions per level and proof: 16, 4 and 1
-# lanes per compression, a warp and a thread per leaf
-@pytest.mark.parametrize("n", [2, 12, 40])
+# about 700 leaves and as many compressions per level and proof: 16, 4 and 1
+# lanes per compression; a warp, four lanes and a thread per leaf
+@pytest.mark.parametrize("n", [2, 5, 40, 320])
 def test_batches_of_every_size_match_single(product, gpu_ctx, n):
     k, t = O.cubic_trace(9, 12, 5)
     pcs = product.PcsParams(2, 1, 1, 3, 1, 100, 2)
