@@ -13,13 +13,14 @@
 //  with f_red(x_i) = sum_m dot(coef_m, M_m[i >> lift_m])
 //  (deep/prover.rs:304-405).
 #pragma once
+#include "context.cuh"
 #include "gl.cuh"
 #include "ntt.cuh"
 
 namespace deep {
 
 constexpr int CHUNK = 8;
-constexpr int MAX_DOTS = 24;  // matrices
+constexpr int MAX_DOTS = 24;  // matrices of a launch
 
 struct PQArgs {
     uint64_t n;
@@ -77,12 +78,17 @@ __global__ void top_weights_kernel(const uint64_t *q, uint64_t d, uint32_t log_n
 #pragma unroll
     for (int k = 0; k < 4; k++) W[4 * i + k] = gl::mul(q[4 * i + k], x);
 }
-// A launch over parts of different sizes: part k has the blocks first[k] <= b <
-// first[k + 1].
+// A launch over parts of different sizes, at most MAX_DOTS: part k has the
+// blocks first[k] <= b < first[k + 1].
 struct Parts {
     int n = 0;
     uint32_t first[MAX_DOTS + 1] = {0};
-    void add(uint64_t blocks) { n++, first[n] = first[n - 1] + (uint32_t)blocks; }
+    int add(uint64_t blocks) {  // the new part's index
+        if (n == MAX_DOTS) throw p3g::CudaError{p3g::ERR_INVALID, "too many parts in one launch"};
+        first[n + 1] = first[n] + (uint32_t)blocks;
+        return n++;
+    }
+    uint32_t blocks() const { return first[n]; }
     __device__ __forceinline__ int find(uint32_t &b) const {  // b: the block within its part
         int k = 0;
         while (k + 1 < n && first[k + 1] <= b) k++;

@@ -486,15 +486,20 @@ inline std::vector<uint64_t> deep_evals(Ctx &ctx, Launcher &L, const std::vector
       ntt::PowTab{twn.fwd_lo.p, twn.fwd_hi.p, twn.lo_bits}, weights[d].p);
     {
         deep::FoldWeightsArgs fa{};
+        auto launch = [&] {
+            fa.Wb = weights[d].p;
+            if (fa.parts.n) L(deep::fold_weights_kernel, fa.parts.blocks(), 256, 0, fa);
+            fa = deep::FoldWeightsArgs{};
+        };
         for (const Mat *m : all) {
             const uint64_t dm = m->h >> lb;
             if (weights.count(dm)) continue;
             weights[dm] = ctx.alloc(4 * dm);
-            fa.n_small[fa.parts.n] = dm, fa.r[fa.parts.n] = d / dm, fa.Ws[fa.parts.n] = weights[dm].p;
-            fa.parts.add(blocks_for(dm * 8, 256));
+            const int k = fa.parts.add(blocks_for(dm * 8, 256));
+            fa.n_small[k] = dm, fa.r[k] = d / dm, fa.Ws[k] = weights[dm].p;
+            if (fa.parts.n == deep::MAX_DOTS) launch();
         }
-        fa.Wb = weights[d].p;
-        if (fa.parts.n) L(deep::fold_weights_kernel, fa.parts.first[fa.parts.n], 256, 0, fa);
+        launch();
     }
     gl::ef sj[2];
     for (int j = 0; j < 2; j++) {
@@ -518,26 +523,28 @@ inline std::vector<uint64_t> deep_evals(Ctx &ctx, Launcher &L, const std::vector
         };
         uint64_t rows = 64;
         while (rows < d && blocks(rows) > target_blocks) rows += (rows + 31) / 32;
-        deep::ColsumArgs ca{};
-        deep::ColsumFinishArgs fa{};
-        ca.rows_per_chunk = rows;
-        fa.s0 = sj[0], fa.s1 = sj[1];
         uint64_t words = 0, off = 0;
         for (const Mat *m : all) words += ((m->h >> lb) + rows - 1) / rows * m->w * 4;
         DBuf part = ctx.alloc(words);
         words = 0;
-        for (size_t mi = 0; mi < all.size(); mi++) {
-            const Mat *m = all[mi];
-            const uint64_t dm = m->h >> lb, n_chunks = (dm + rows - 1) / rows;
-            ca.M[mi] = m->d, ca.W[mi] = weights[dm].p, ca.w[mi] = fa.w[mi] = m->w, ca.d[mi] = dm;
-            ca.partial[mi] = part.p + words, fa.partial[mi] = part.p + words;
-            fa.n_chunks[mi] = n_chunks, fa.out[mi] = evals.p + 4 * off;
-            ca.parts.add((m->w + 31) / 32 * n_chunks);
-            fa.parts.add(blocks_for(m->w * 4, 32));
-            words += n_chunks * m->w * 4, off += m->w;
+        for (size_t first = 0; first < all.size(); first += deep::MAX_DOTS) {  // matrices of a launch
+            deep::ColsumArgs ca{};
+            deep::ColsumFinishArgs fa{};
+            ca.rows_per_chunk = rows;
+            fa.s0 = sj[0], fa.s1 = sj[1];
+            for (size_t mi = first; mi < std::min(all.size(), first + deep::MAX_DOTS); mi++) {
+                const Mat *m = all[mi];
+                const uint64_t dm = m->h >> lb, n_chunks = (dm + rows - 1) / rows;
+                const int k = ca.parts.add((m->w + 31) / 32 * n_chunks);
+                fa.parts.add(blocks_for(m->w * 4, 32));
+                ca.M[k] = m->d, ca.W[k] = weights[dm].p, ca.w[k] = fa.w[k] = m->w, ca.d[k] = dm;
+                ca.partial[k] = part.p + words, fa.partial[k] = part.p + words;
+                fa.n_chunks[k] = n_chunks, fa.out[k] = evals.p + 4 * off;
+                words += n_chunks * m->w * 4, off += m->w;
+            }
+            L(deep::colsum_kernel, ca.parts.blocks(), 256, 0, ca);
+            L(deep::colsum_finish_kernel, fa.parts.blocks(), 512, 0, fa);
         }
-        L(deep::colsum_kernel, ca.parts.first[all.size()], 256, 0, ca);
-        L(deep::colsum_finish_kernel, fa.parts.first[all.size()], 512, 0, fa);
     }
     std::vector<uint64_t> h_evals(4 * total_w);
     ctx.d2h(h_evals.data(), evals.p, 4 * total_w);
