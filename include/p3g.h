@@ -324,9 +324,11 @@ int p3g_ctx_set_slab_columns(p3g_ctx *ctx, uint64_t cols);
 /* No counterpart in the reference: the context's memory pool, bytes reserved
  * from the device and in use, and the host time spent in allocation calls
  * since creation (growth of the pool maps device memory inside them). */
-/* No counterpart in the reference: DAG nodes per generated constraint kernel
- * for symbolic AIRs created on this context afterwards (0: default 500;
- * otherwise at least 16). Results do not depend on it. */
+/* No counterpart in the reference: bound on the DAG nodes (operations and
+ * trace cells) of a generated constraint kernel for symbolic AIRs created on
+ * this context afterwards; a constraint above it is a kernel alone. 0: the
+ * default, 500, and 1024 where one group of constraints that share their
+ * cells needs more; otherwise at least 16. Results do not depend on it. */
 int p3g_ctx_set_air_chunk_nodes(p3g_ctx *ctx, uint64_t nodes);
 int p3g_ctx_memory_stats(p3g_ctx *ctx, uint64_t *reserved_bytes, uint64_t *used_bytes, double *alloc_ms);
 

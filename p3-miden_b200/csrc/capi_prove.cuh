@@ -583,7 +583,7 @@ P3G_API int p3g_air_create(p3g_ctx *x, const p3g_air_desc_c *desc, p3g_sym_air *
     try {
         CK(cudaSetDevice(x->c.device));
         sym::analyse(a->a);
-        if (x->c.air_chunk_nodes) a->a.chunk_nodes = x->c.air_chunk_nodes;
+        if (x->c.air_chunk_nodes) a->a.chunk_nodes = a->a.group_nodes = x->c.air_chunk_nodes;
         sym::split_chunks(a->a);
         sym::compile(a->a, x->c.device);
     } catch (const p3g::CudaError &e) {

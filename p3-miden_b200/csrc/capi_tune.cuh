@@ -172,9 +172,10 @@ P3G_API int p3g_ctx_set_slab_columns(p3g_ctx *x, uint64_t cols) {
     x->c.slab_cols = cols;
     return p3g::OK;
 }
-// DAG nodes per generated constraint kernel for the symbolic AIRs this
-// context creates afterwards (0 restores the default). Fewer nodes: shorter
-// kernels (instruction cache) but more launches re-reading shared cells.
+// Bound on the DAG nodes of a generated constraint kernel for the symbolic
+// AIRs this context creates afterwards (0 restores the defaults; a larger
+// constraint is a kernel alone). Fewer nodes: shorter kernels (instruction
+// cache) but more launches re-reading shared cells.
 P3G_API int p3g_ctx_set_air_chunk_nodes(p3g_ctx *x, uint64_t nodes) {
     if (!x || (nodes && nodes < 16)) return p3g::ERR_INVALID;
     x->c.air_chunk_nodes = nodes;

@@ -145,8 +145,8 @@ struct Ctx {
     // them: every choice computes the same values.
     std::map<uint32_t, std::vector<uint32_t>> lde_split;
     uint64_t slab_cols = 0;
-    // DAG nodes per generated constraint kernel of the symbolic AIRs created
-    // on this context (0: the default, 500)
+    // bound on the DAG nodes of a generated constraint kernel of the symbolic
+    // AIRs created on this context (0: the defaults of sym::Air)
     uint64_t air_chunk_nodes = 0;
 
     // Tables of the tensor-core permutation (p2tc.cuh) for this context's

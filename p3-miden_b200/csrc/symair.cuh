@@ -37,8 +37,9 @@
 #include <cstring>
 #include <mutex>
 #include <sstream>
-#include <thread>
 #include <string>
+#include <thread>
+#include <unordered_set>
 #include <vector>
 
 #include "context.cuh"
@@ -90,7 +91,9 @@ struct Air {
     std::vector<uint64_t> base_idx, ext_idx;  // ConstraintLayout
     KLayout kl;
     std::vector<std::vector<ChunkGroup>> chunks;  // constraints of each generated kernel
-    size_t chunk_nodes = 500;  // DAG nodes per chunk (a launch-shape choice; every value gives the same sums)
+    // bounds on a chunk's DAG nodes, packed from groups and of one group (a
+    // launch-shape choice; every value gives the same sums)
+    size_t chunk_nodes = 500, group_nodes = 1024;
     std::string source, log;
     std::vector<std::vector<char>> cubins;  // one per compiled group of chunks
     std::vector<cudaLibrary_t> libs;
@@ -214,12 +217,10 @@ struct KArgs {
     uint64_t *acc;         // EF accumulator, += the folded numerator
 };
 
-// Constraints are split into chunks of bounded code size (about
-// A.chunk_nodes DAG nodes each, shared subexpressions counted once per chunk);
-// each chunk is one kernel that adds its part of the fold into acc. The fold
-// is linear, so launching the chunks one after another on the same stream
-// gives the same sum, in any order of the constraints. A small AIR is one
-// chunk.
+// Constraints are split into chunks, one kernel each that adds its part of the
+// fold into acc. The fold is linear, so launching the chunks one after another
+// on the same stream gives the same sum, in any order of the constraints. A
+// small AIR is one chunk.
 //
 // A cell that two chunks read is loaded from HBM twice, and a subexpression
 // two chunks need is evaluated twice, so constraints are first grouped by what
@@ -230,6 +231,14 @@ struct KArgs {
 // is live; and the small constraints (booleans, parities) whose cells a group
 // loads follow as soon as their last cell is there. In emission order the
 // Keccak AIR's chunks loaded 14.6 k cells per point, 5.5 times its columns.
+//
+// Code size is bounded, as a kernel compiles on one thread in a time that
+// grows faster than linearly (1401 nodes 7 s, 5620 nodes 129 s): a group takes
+// a constraint only while its operations and cells stay within group_nodes,
+// and groups share a chunk only within chunk_nodes, shared nodes counted once.
+// One constraint above the bounds is a chunk alone. group_nodes: the Keccak
+// AIR's largest group has 1014; chunk_nodes: its constraint stage took 15.07
+// ms at 500, 15.74 at 800 and 17.2 at 1200 (2^18 rows).
 constexpr size_t kGroupMax = 5, kSmallNodes = 40;
 
 inline void split_chunks(Air &A) {
@@ -274,12 +283,15 @@ inline void split_chunks(Air &A) {
         ChunkGroup g;
         touched.clear();
         uint32_t add = (uint32_t)k;
+        const uint32_t mine = (uint32_t)(nc + 1 + k);  // marks the group's nodes
+        size_t held = 0;
         for (;;) {
             g.step.push_back(add);
             placed[add] = 1;
             for (uint32_t i : nodes[add]) {
-                if (seen[i] == nc + 1 + k) continue;  // counted for this group
-                seen[i] = (uint32_t)(nc + 1 + k);
+                if (seen[i] == mine) continue;  // counted for this group
+                seen[i] = mine;
+                held++;
                 if (readers[i].size() > kCommon) continue;
                 for (uint32_t u : readers[i]) {
                     if (placed[u]) continue;
@@ -294,19 +306,27 @@ inline void split_chunks(Air &A) {
                     (best < 0 || shared[u] > shared[best] || (shared[u] == shared[best] && u < best)))
                     best = u;
             if (best < 0) break;
+            size_t fresh = 0;
+            for (uint32_t i : nodes[best]) fresh += seen[i] != mine;
+            if (held + fresh > A.group_nodes) break;
             add = (uint32_t)best;
         }
         for (uint32_t u : touched) shared[u] = 0;
         groups.push_back(std::move(g));
     }
-    // small constraints: to the first group that loads all their cells
-    std::vector<int64_t> cell_group(n, -1);  // last group seen loading the cell
+    // small constraints: to the first group that loads all their cells and has
+    // room for their other nodes
+    std::vector<std::unordered_set<uint32_t>> held(groups.size());
     std::vector<std::vector<uint32_t>> cell_groups(n);
     for (size_t g = 0; g < groups.size(); g++)
         for (uint32_t k : groups[g].step)
             for (uint32_t i : nodes[k])
-                if (is_cell(d.nodes[i]) && cell_group[i] != (int64_t)g)
-                    cell_group[i] = (int64_t)g, cell_groups[i].push_back((uint32_t)g);
+                if (held[g].insert(i).second && is_cell(d.nodes[i])) cell_groups[i].push_back((uint32_t)g);
+    auto room = [&](size_t g, uint32_t k) {
+        size_t fresh = 0;
+        for (uint32_t i : nodes[k]) fresh += !held[g].count(i);
+        return held[g].size() + fresh <= A.group_nodes;
+    };
     std::vector<uint32_t> hits(groups.size(), 0);
     std::vector<ChunkGroup> rest;
     for (size_t k = 0; k < nc; k++) {
@@ -322,11 +342,12 @@ inline void split_chunks(Air &A) {
                     if (hits[g]++ == 0) touched.push_back(g);
             }
         for (uint32_t g : touched) {
-            if (cells && hits[g] == cells && (home < 0 || g < home)) home = g;
+            if (cells && hits[g] == cells && (home < 0 || g < home) && room(g, (uint32_t)k)) home = g;
             hits[g] = 0;
         }
         if (home >= 0) {
             groups[home].small.push_back((uint32_t)k);
+            held[home].insert(nodes[k].begin(), nodes[k].end());
         } else {
             rest.emplace_back();
             rest.back().step.push_back((uint32_t)k);
