@@ -215,11 +215,13 @@ struct DeepArgs {
     int32_t *flags;            // flags[0]: a denominator vanished
 };
 // One warp per query: red_row = sum_i v_i * alpha_c^(T-1-i), then
-// de = sum_p bp^p (red_open_p - red_row) / (z_p - x_q). Proof blockIdx.y (all
-// proofs of a pass in one launch; one after another they took 20 us each).
-__global__ void __launch_bounds__(128) deep_kernel(const DeepArgs *args) {
-    const DeepArgs &a = args[blockIdx.y];
-    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// de = sum_p bp^p (red_open_p - red_row) / (z_p - x_q). All proofs of a pass in
+// one launch (one after another they took 20 us each), `per` blocks each on
+// the grid's x: y ends at 65,535.
+__global__ void __launch_bounds__(128) deep_kernel(const DeepArgs *args, uint32_t per) {
+    const uint32_t proof = blockIdx.x / per;
+    const DeepArgs &a = args[proof];
+    const uint32_t q = ((blockIdx.x - proof * per) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (q >= a.nq) return;
     gl::Acc c0, c1;
@@ -937,8 +939,8 @@ inline void device_pass(Ctx &ctx, const std::vector<Prepared *> &vs, Timing *tm,
         launch_compress(ctx, (const CJob *)(d.p + o_cj) + lv_off[l], (uint32_t)(lv_off[l + 1] - lv_off[l]), pool);
     }
     if (n_deep) {
-        deep_kernel<<<dim3((unsigned)((max_nq * 32 + 127) / 128), (unsigned)n_deep), 128, 0, ctx.stream>>>(
-            (const DeepArgs *)(d.p + o_das));
+        const unsigned per = (unsigned)((max_nq * 32 + 127) / 128);
+        deep_kernel<<<(unsigned)n_deep * per, 128, 0, ctx.stream>>>((const DeepArgs *)(d.p + o_das), per);
         CK(cudaGetLastError());
         ctx.launches++;
     }
