@@ -34,7 +34,7 @@ enum p3g_status {
     P3G_ERR_INVALID = 1,    /* bad argument: null pointer, size, unsupported parameter */
     P3G_ERR_VALIDATION = 2, /* ProverError / AirValidationError equivalents */
     P3G_ERR_OOM = 3,        /* device allocation refused */
-    P3G_ERR_TIMEOUT = 4,    /* a bounded search gave up (proof-of-work) */
+    P3G_ERR_TIMEOUT = 4,    /* a bounded search (proof-of-work) or device-side wait gave up */
     P3G_ERR_CUDA = 5,       /* other CUDA runtime error */
     P3G_ERR_REJECTED = 6    /* a served proof failed the server's self-check (p3g_server_set_self_check) */
 };
@@ -330,6 +330,11 @@ int p3g_ctx_set_slab_columns(p3g_ctx *ctx, uint64_t cols);
  * default, 500, and 1024 where one group of constraints that share their
  * cells needs more; otherwise at least 16. Results do not depend on it. */
 int p3g_ctx_set_air_chunk_nodes(p3g_ctx *ctx, uint64_t nodes);
+/* No counterpart in the reference: how long the hash kernels of large classes
+ * wait for one product of the tensor cores (about a microsecond); a wait that
+ * runs out ends the call with P3G_ERR_TIMEOUT, and the context stays usable.
+ * ns: from 0 (every wait gives up at once) to 100,000,000 (the default). */
+int p3g_ctx_set_hash_wait(p3g_ctx *ctx, uint32_t ns);
 int p3g_ctx_memory_stats(p3g_ctx *ctx, uint64_t *reserved_bytes, uint64_t *used_bytes, double *alloc_ms);
 
 /* ------------------------------------------------------------ verifier */

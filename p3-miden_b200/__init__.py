@@ -171,6 +171,7 @@ def lib():
             "p3g_air_num_constraints_of": (C.c_uint64, [vp]),
             "p3g_air_num_kernels": (C.c_uint64, [vp]),
             "p3g_ctx_set_air_chunk_nodes": (C.c_int, [vp, C.c_uint64]),
+            "p3g_ctx_set_hash_wait": (C.c_int, [vp, C.c_uint32]),
             "p3g_air_layout": (C.c_int, [vp, u64p, C.POINTER(C.c_uint64), u64p, C.POINTER(C.c_uint64)]),
             "p3g_air_free": (None, [vp]),
         }
@@ -269,6 +270,11 @@ class Context:
         """DAG nodes per generated constraint kernel of symbolic AIRs created
         on this context from now on (0: the default)."""
         self.check(lib().p3g_ctx_set_air_chunk_nodes(self._h, nodes))
+
+    def set_hash_wait(self, ns: int):
+        """How long the hash kernels wait for a product of the tensor cores
+        before the call ends with ERR_TIMEOUT (0..10^8 ns, the default)."""
+        self.check(lib().p3g_ctx_set_hash_wait(self._h, ns))
 
     def memory_stats(self) -> dict:
         """The context pool's reserved and used bytes, and the host ms spent in

@@ -182,6 +182,14 @@ P3G_API int p3g_ctx_set_air_chunk_nodes(p3g_ctx *x, uint64_t nodes) {
     return p3g::OK;
 }
 
+// Nanoseconds that a hash kernel waits for the tensor cores before it gives up
+// and the call returns P3G_ERR_TIMEOUT (at most the default, 0.1 s).
+P3G_API int p3g_ctx_set_hash_wait(p3g_ctx *x, uint32_t ns) {
+    if (!x || ns > p2t::kWaitNs) return p3g::ERR_INVALID;
+    x->c.hash_wait_ns = ns;
+    return p3g::OK;
+}
+
 // Memory statistics of the context's pool: bytes reserved from the device,
 // bytes in use by live buffers, and the host time spent in allocation calls
 // since the context was created (a pool that grows maps new device memory

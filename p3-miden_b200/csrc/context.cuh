@@ -28,7 +28,7 @@ enum Status : int {
     ERR_INVALID = 1,     // bad argument (null pointer, size, unsupported parameter)
     ERR_VALIDATION = 2,  // instance validation failed (AIR, height order, width)
     ERR_OOM = 3,         // device allocation refused
-    ERR_TIMEOUT = 4,     // a bounded device-side search gave up
+    ERR_TIMEOUT = 4,     // a bounded device-side search or wait gave up
     ERR_CUDA = 5,        // other CUDA runtime error
     ERR_REJECTED = 6,    // the server's self-check rejected the proof
 };
@@ -163,7 +163,8 @@ struct Ctx {
         *hash_err = 0;
         hash_table = upload(words);
     }
-    p2t::Args hash_args() const { return p2t::Args{(const uint8_t *)hash_table.p, hash_err}; }
+    uint32_t hash_wait_ns = p2t::kWaitNs;  // p3g_ctx_set_hash_wait
+    p2t::Args hash_args() const { return p2t::Args{(const uint8_t *)hash_table.p, hash_err, hash_wait_ns}; }
 
     // This context's own stream-ordered memory pool. Buffers freed by one
     // context are reused only by that context, so two contexts driving the

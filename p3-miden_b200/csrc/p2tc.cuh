@@ -110,9 +110,12 @@ inline bool build_tables(const uint64_t *c, std::vector<uint8_t> &img) {
     return worst * 255 * 257 < (1ull << 32);
 }
 
+// A wait gives up after 0.1 s; a product takes about a microsecond.
+constexpr uint32_t kWaitNs = 100000000;
 struct Args {
     const uint8_t *table;  // kTableBytes, device
     uint32_t *err;         // set when a wait gave up
+    uint32_t wait_ns;      // kWaitNs, or less; 0: every wait gives up at once
 };
 
 // One group's handles.
@@ -127,6 +130,7 @@ struct Group {
     bool dead;
     uint8_t *my_row;   // this thread's 16-byte column of y rows
     uint32_t *err;
+    uint32_t wait_ns;
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -148,15 +152,47 @@ __device__ __forceinline__ void ld16(uint32_t a, uint32_t *v) {
                  : "r"(a)
                  : "memory");
 }
+// One poll; with SUSPEND the hardware may hold the thread for some time first.
+template <bool SUSPEND = true>
 __device__ __forceinline__ bool try_wait(uint32_t mbar, uint32_t phase) {
     uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(mbar), "r"(phase)
-                 : "memory");
+    if (SUSPEND)
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(mbar), "r"(phase)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(mbar), "r"(phase)
+                     : "memory");
     return ok != 0;
+}
+
+__device__ __forceinline__ uint64_t now_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// Whether the phase ends within ns. kGrace more polls come after the time is
+// up (a fraction of a millisecond), so that a context switch in between, after
+// which the group's other warps still have to reach the barrier, does not
+// count as a wait.
+constexpr int kGrace = 4096;
+__device__ __forceinline__ bool wait(uint32_t mbar, uint32_t phase, uint32_t ns) {
+    if (ns == 0) return false;
+    if (try_wait(mbar, phase)) return true;
+    const uint64_t t0 = now_ns();
+    while (now_ns() - t0 < ns)
+        if (try_wait(mbar, phase)) return true;
+#pragma unroll 1
+    for (int i = 0; i < kGrace; i++)
+        if (try_wait<false>(mbar, phase)) return true;
+    return false;
 }
 
 // Tables, barriers, TMEM and the constant word; every thread of the CTA.
@@ -191,6 +227,7 @@ __device__ __forceinline__ Group setup(uint8_t *smem, const Args &a) {
     g.warp = warp;
     g.dead = false;
     g.err = a.err;
+    g.wait_ns = a.wait_ns;
     st4(g.tm, 1, 0);
     return g;
 }
@@ -203,15 +240,19 @@ __device__ __forceinline__ void teardown(Group &g) {
 }
 
 // Batch `batch` over the y rows and the first 4 * z_steps words of the z
-// part; the whole group calls it. One warp collects the others and one of its
-// threads issues; the group's earlier accesses to its operands are complete.
-// The warps take turns (a batch is about 75 instructions to issue): with the
+// part; the whole group calls it, and one thread issues once the group's
+// earlier accesses to its operands are complete. All four warps wait at the
+// barrier, although only the issuing one needs the others: threads that gave up
+// are not paced by the batches any more, and with bare arrivals one warp's next
+// could complete this batch's barrier in another's place and leave a third
+// waiting for good (this costs 0.2 to 0.6 %: a 2^18 x 336 slab's commit 12.95
+// against 12.88 ms). The warps take turns (a batch is about 75 instructions to issue): with the
 // same warp of every group, that scheduler alone had 10 % more to do, 1.79
 // against 1.91 G permutations/s.
 __device__ __forceinline__ void issue(Group &g, int batch, int z_steps) {
     fence_before();
+    asm volatile("bar.sync %0, 128;" ::"r"(g.bar) : "memory");
     if (((batch + g.bar) & 3) == g.warp) {
-        asm volatile("bar.sync %0, 128;" ::"r"(g.bar) : "memory");
         if ((threadIdx.x & 31) == 0 && !g.dead) {
             fence_after();
             const uint32_t tm = g.tm & 0xFFFF;  // lane 0
@@ -237,19 +278,21 @@ __device__ __forceinline__ void issue(Group &g, int batch, int z_steps) {
                          : "memory");
         }
         __syncwarp();
-    } else {
-        asm volatile("bar.arrive %0, 128;" ::"r"(g.bar) : "memory");
     }
 }
 // Waits for the batch in flight and reads its two outputs' accumulators. A
-// wait that runs out marks the launch as failed (the host checks err) and
-// the group goes on without waiting, to a bounded end.
+// wait that runs out marks the launch as failed (the host checks err), and the
+// thread neither issues nor waits for a further batch, but keeps to the group's
+// barriers, to a bounded end (a batch that is not issued makes the other
+// threads' waits run out too). It goes on only after a second bounded wait for
+// the batch itself, which would otherwise read shared memory and write TMEM
+// that the CTA has given back: every batch is waited for by the warp that
+// issued it, so none is in flight at teardown.
 __device__ __forceinline__ void collect(Group &g, uint32_t *L) {
-    bool ok = g.dead;
-    for (int i = 0; i < (1 << 16) && !ok; i++) ok = try_wait(g.mbar, g.phase);
-    if (!ok) {
+    if (!g.dead && !wait(g.mbar, g.phase, g.wait_ns)) {
         *g.err = 1;
         g.dead = true;
+        wait(g.mbar, g.phase, kWaitNs);
     }
     g.phase ^= 1;
     __syncwarp();
