@@ -127,9 +127,8 @@ P3G_API int p3g_prove(p3g_ctx *x, const p3g_pcs_params_c *pcs, const p3g_instanc
         x->c.last_error = "instance or parameter validation failed";
         return v;
     }
-    try {
+    P3G_TRY(x, {
         CK(cudaSetDevice(x->c.device));
-        p3g::bind_p2(x->c);
         p3g::ensure_keccak_tables(x->c.device);
         std::vector<p3g::Instance> ins(n);
         for (uint64_t i = 0; i < n; i++) ins[i] = p3g::to_instance(inst[i]);
@@ -149,14 +148,7 @@ P3G_API int p3g_prove(p3g_ctx *x, const p3g_pcs_params_c *pcs, const p3g_instanc
         out->gpu_launches = po.launches;
         out->h2d_bytes = po.h2d;
         out->d2h_bytes = po.d2h;
-    } catch (const p3g::CudaError &e) {
-        x->c.last_error = e.what;
-        return e.status;
-    } catch (const std::bad_alloc &) {
-        x->c.last_error = "host allocation failed";
-        return p3g::ERR_OOM;
-    }
-    return p3g::OK;
+    })
 }
 
 // Wire format of a proof (StarkOutput: digest + TranscriptData,

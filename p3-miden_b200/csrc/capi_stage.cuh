@@ -18,9 +18,11 @@ struct p3g_tree {
         __VA_ARGS__;                                          \
         return p3g::OK;                                       \
     } catch (const p3g::CudaError &e) {                       \
+        if (ctxp) (ctxp)->c.recover();                        \
         if (ctxp) (ctxp)->c.last_error = e.what;              \
         return e.status;                                      \
     } catch (const std::bad_alloc &) {                        \
+        if (ctxp) (ctxp)->c.recover();                        \
         if (ctxp) (ctxp)->c.last_error = "host allocation failed"; \
         return p3g::ERR_OOM;                                  \
     }
@@ -102,21 +104,15 @@ P3G_API int p3g_lmcs_build(p3g_ctx *x, const uint64_t *const *d_mats, const uint
         if (i && heights[i] < heights[i - 1]) return p3g::ERR_VALIDATION;
     }
     *out = nullptr;
-    p3g_tree *t = new p3g_tree();
-    try {
+    P3G_TRY(x, {
         CK(cudaSetDevice(x->c.device));
-        p3g::bind_p2(x->c);
+        auto t = std::make_unique<p3g_tree>();
         std::vector<p3g::Mat> mats;
         for (uint64_t i = 0; i < n; i++) mats.push_back({d_mats[i], heights[i], widths[i]});
         p3g::build_tree(x->c, t->t, mats, alignment);
         x->c.sync();
-    } catch (const p3g::CudaError &e) {
-        x->c.last_error = e.what;
-        delete t;
-        return e.status;
-    }
-    *out = t;
-    return p3g::OK;
+        *out = t.release();
+    })
 }
 
 // HidingLmcsConfig::build_tree / build_aligned_tree
@@ -133,22 +129,16 @@ P3G_API int p3g_lmcs_build_hiding(p3g_ctx *x, const uint64_t *const *d_mats, con
         if (i && heights[i] < heights[i - 1]) return p3g::ERR_VALIDATION;
     }
     *out = nullptr;
-    p3g_tree *t = new p3g_tree();
-    try {
+    P3G_TRY(x, {
         CK(cudaSetDevice(x->c.device));
-        p3g::bind_p2(x->c);
+        auto t = std::make_unique<p3g_tree>();
         std::vector<p3g::Mat> mats;
         for (uint64_t i = 0; i < n; i++) mats.push_back({d_mats[i], heights[i], widths[i]});
         const p3g::Mat salt{d_salt, heights[n - 1], salt_width};
         p3g::build_tree(x->c, t->t, mats, alignment, &salt);
         x->c.sync();
-    } catch (const p3g::CudaError &e) {
-        x->c.last_error = e.what;
-        delete t;
-        return e.status;
-    }
-    *out = t;
-    return p3g::OK;
+        *out = t.release();
+    })
 }
 
 P3G_API int p3g_lmcs_root(const p3g_tree *t, uint64_t *out4) {

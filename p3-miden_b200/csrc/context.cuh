@@ -276,6 +276,14 @@ struct Ctx {
             throw CudaError{ERR_TIMEOUT, "hash kernel: a tensor-core wait ran out"};
         }
     }
+    // After a call that failed: what it started ends before the caller has its
+    // buffers back, and a hash kernel that gave up in it does not fail the next
+    // call's sync.
+    void recover() {
+        for (cudaStream_t s : {copy_stream, lde_stream, stream})
+            if (s) cudaStreamSynchronize(s);
+        if (hash_err) *hash_err = 0;
+    }
     // upload a small host vector to a fresh device buffer
     DBuf upload(const std::vector<uint64_t> &v) {
         DBuf b = alloc(v.size());

@@ -217,11 +217,12 @@ class Server {
             } catch (const CudaError &e) {
                 st = e.status;
                 job->error = e.what;
-                cudaStreamSynchronize(ctx.stream);
+                ctx.recover();
                 cudaGetLastError();
             } catch (const std::bad_alloc &) {
                 st = ERR_OOM;
                 job->error = "host allocation failed";
+                ctx.recover();
             }
             // the workspace is part of the job's footprint: give it back to the
             // worker's pool, which keeps memory only within its budget share
