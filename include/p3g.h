@@ -330,6 +330,11 @@ int p3g_ctx_set_slab_columns(p3g_ctx *ctx, uint64_t cols);
  * default, 500, and 1024 where one group of constraints that share their
  * cells needs more; otherwise at least 16. Results do not depend on it. */
 int p3g_ctx_set_air_chunk_nodes(p3g_ctx *ctx, uint64_t nodes);
+/* No counterpart in the reference: whether large classes and levels hash on
+ * the tensor cores (default 1) or one thread per state, as they do with a
+ * Poseidon2 table whose products do not fit 32 bits there. Results do not
+ * depend on it. */
+int p3g_ctx_set_tensor_hash(p3g_ctx *ctx, int32_t enabled);
 /* No counterpart in the reference: how long the hash kernels of large classes
  * wait for one product of the tensor cores (about a microsecond); a wait that
  * runs out ends the call with P3G_ERR_TIMEOUT, and the context stays usable.

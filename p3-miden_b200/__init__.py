@@ -172,6 +172,7 @@ def lib():
             "p3g_air_num_kernels": (C.c_uint64, [vp]),
             "p3g_ctx_set_air_chunk_nodes": (C.c_int, [vp, C.c_uint64]),
             "p3g_ctx_set_hash_wait": (C.c_int, [vp, C.c_uint32]),
+            "p3g_ctx_set_tensor_hash": (C.c_int, [vp, C.c_int32]),
             "p3g_air_layout": (C.c_int, [vp, u64p, C.POINTER(C.c_uint64), u64p, C.POINTER(C.c_uint64)]),
             "p3g_air_free": (None, [vp]),
         }
@@ -270,6 +271,11 @@ class Context:
         """DAG nodes per generated constraint kernel of symbolic AIRs created
         on this context from now on (0: the default)."""
         self.check(lib().p3g_ctx_set_air_chunk_nodes(self._h, nodes))
+
+    def set_tensor_hash(self, enabled: bool):
+        """Whether large classes and levels hash on the tensor cores (the
+        default) or one thread per state; results do not depend on it."""
+        self.check(lib().p3g_ctx_set_tensor_hash(self._h, int(enabled)))
 
     def set_hash_wait(self, ns: int):
         """How long the hash kernels wait for a product of the tensor cores

@@ -182,6 +182,14 @@ P3G_API int p3g_ctx_set_air_chunk_nodes(p3g_ctx *x, uint64_t nodes) {
     return p3g::OK;
 }
 
+// Whether classes and levels large enough for it hash on the tensor cores
+// (the default); if not, one thread per state as with constants that do not
+// fit the byte tables.
+P3G_API int p3g_ctx_set_tensor_hash(p3g_ctx *x, int32_t enabled) {
+    if (!x) return p3g::ERR_INVALID;
+    x->c.tensor_hash = enabled != 0;
+    return p3g::OK;
+}
 // Nanoseconds that a hash kernel waits for the tensor cores before it gives up
 // and the call returns P3G_ERR_TIMEOUT (at most the default, 0.1 s).
 P3G_API int p3g_ctx_set_hash_wait(p3g_ctx *x, uint32_t ns) {

@@ -164,6 +164,8 @@ struct Ctx {
         hash_table = upload(words);
     }
     uint32_t hash_wait_ns = p2t::kWaitNs;  // p3g_ctx_set_hash_wait
+    bool tensor_hash = true;                // p3g_ctx_set_tensor_hash
+    bool use_tensor_hash() const { return tensor_hash && hash_table.p; }
     p2t::Args hash_args() const { return p2t::Args{(const uint8_t *)hash_table.p, hash_err, hash_wait_ns}; }
 
     // This context's own stream-ordered memory pool. Buffers freed by one
@@ -723,7 +725,7 @@ inline void launch_leaf_class(Ctx &ctx, const merkle::ClassArgs &a, uint64_t n) 
         const unsigned quad_blocks = (unsigned)((n * 4 + 127) / 128);
         if (a.cm) merkle::leaf_class_quad_kernel<true><<<quad_blocks, 128, 0, ctx.stream>>>(a);
         else merkle::leaf_class_quad_kernel<false><<<quad_blocks, 128, 0, ctx.stream>>>(a);
-    } else if (n >= kTcLeaves && ctx.hash_table.p) {
+    } else if (n >= kTcLeaves && ctx.use_tensor_hash()) {
         uint64_t perms = 0;
         for (int m = 0; m < a.n_mats; m++) perms += (a.width[m] + 7) / 8;
         static std::atomic<uint64_t> attr_cm{0}, attr{0};
@@ -749,7 +751,7 @@ inline void launch_leaf_class(Ctx &ctx, const merkle::ClassArgs &a, uint64_t n) 
 constexpr uint64_t kWideParents = 1ull << 14, kTcParents = 1ull << 16, kQuadParents = 1ull << 12;
 inline void compress_layers(Ctx &ctx, Tree &t) {
     uint32_t l = 0;
-    for (; ctx.hash_table.p && l < t.depth && (t.H >> (l + 1)) >= kTcParents; l++) {
+    for (; ctx.use_tensor_hash() && l < t.depth && (t.H >> (l + 1)) >= kTcParents; l++) {
         static std::atomic<uint64_t> attr{0};
         launch_tc(ctx, attr, merkle::compress_level_tc_kernel, t.H >> (l + 1), 1, t.layers.p, t.H, l);
     }
