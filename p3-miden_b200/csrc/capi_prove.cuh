@@ -300,7 +300,7 @@ P3G_API int p3g_grind(p3g_ctx *x, const uint64_t *state12, const uint64_t *pendi
                 g.base = base;
                 g.count = 1ull << 22;
                 g.found = (unsigned long long *)fb.p;
-                ::fri::grind_kernel<<<148 * ::fri::kGrindBlocks, 128, 0, x->c.stream>>>(g);
+                ::fri::grind_kernel<<<::fri::grind_grid(bits), 128, 0, x->c.stream>>>(g);
                 CK(cudaGetLastError());
                 x->c.d2h(x->c.stage(1), fb.p, 1);
                 x->c.sync();

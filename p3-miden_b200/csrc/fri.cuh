@@ -280,11 +280,14 @@ struct WitnessFound {
 };
 // Candidates are tried in order, a grid's worth at a time, so that the least
 // witness is found. Bound by the latency of a permutation and its integer
-// pipes. Two blocks per SM: a turn of 38 k candidates takes 36 us, and more
-// blocks try more candidates past the least witness (16 bits, mean of 300
-// states with the call: 1 / 2 / 3 / 4 / 8 blocks 133 / 109 / 115 / 125 / 158
-// us; 130 us with two when a turn begun beside the find ran to its end).
-constexpr int kGrindBlocks = 2;
+// pipes. Two blocks per SM while a search is a few turns: a turn of 38 k
+// candidates takes 36 us, and more blocks try more candidates past the least
+// witness (16 bits, mean of 300 states with the call: 1 / 2 / 3 / 4 / 8 blocks
+// 133 / 109 / 115 / 125 / 158 us; 130 us with two when a turn begun beside the
+// find ran to its end). A long search is bound by the pipes, which two blocks
+// do not fill: 21 / 22 / 23 / 24 / 26 bits take 2.22 / 4.22 / 9.43 / 12.8 / 80.3
+// ms with two and 2.29 / 3.99 / 8.34 / 11.1 / 67.9 with eight.
+inline unsigned grind_grid(uint32_t bits) { return 148 * (bits < 22 ? 2 : 8); }
 __global__ void __launch_bounds__(128) grind_kernel(const __grid_constant__ GrindArgs a) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t mask = (1ull << a.bits) - 1;

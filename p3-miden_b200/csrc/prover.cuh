@@ -866,7 +866,7 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
             g.base = base;
             g.count = batch;
             g.found = (unsigned long long *)fb.p;
-            L(fri::grind_kernel, 148 * fri::kGrindBlocks, 128, 0, g);
+            L(fri::grind_kernel, fri::grind_grid(g.bits), 128, 0, g);
             ctx.d2h(ctx.stage(1), fb.p, 1);
             ctx.sync();
             found = ctx.pinned[0];
@@ -945,7 +945,7 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
             g.found = found;
             g.ch = devch + r;
             g.root = root;
-            L(fri::grind_kernel, 148 * fri::kGrindBlocks, 128, 0, g);
+            L(fri::grind_kernel, fri::grind_grid(g.bits), 128, 0, g);
         }
         const fri::RoundArgs ra{devch + r, devch + r + 1, root, fbits, found, droots.p + 4 * r, dwit.p + r, dbeta.p + 2 * r};
         const uint64_t nout = dom / arity;
