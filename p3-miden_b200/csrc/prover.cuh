@@ -146,11 +146,15 @@ __global__ void gather_kernel(const Seg *segs, uint64_t n, uint64_t *out) {
 }
 // The segments' words, padded, one behind the other, into host memory: one
 // gather and one copy per 2^24 words (openings are hundreds of rows and
-// digests; a copy each took about 10 us). Memory of another device than the
-// context's, which a kernel here may not reach, is copied piece by piece.
+// digests; a copy each takes about 10 us, the gather of any number 40 to 50).
+// One or two segments, and memory of another device than the context's, which
+// a kernel here may not reach, are copied piece by piece: an opening of one row
+// and one digest takes 39 us so, 78 gathered; three and more gain nothing or
+// lose (one row and four digests 58 and 70 us).
 inline void gather_to_host(Ctx &ctx, std::vector<Seg> &segs, uint64_t *host, int device) {
     constexpr uint64_t kWords = 1ull << 24;
-    if (device != ctx.device) {
+    if (segs.empty()) return;
+    if (device != ctx.device || segs.size() <= 2) {
         for (const Seg &g : segs) {
             ctx.d2h(host, g.src, g.len);
             for (uint64_t k = g.len; k < g.padded; k++) host[k] = 0;
