@@ -114,6 +114,8 @@ inline int validate(const p3g_pcs_params_c *pcs, const p3g_instance_c *inst, uin
     if (log_qd > pcs->log_blowup) return ERR_VALIDATION;  // ConstraintDegreeTooHigh
     if (log_qd > 3) return ERR_VALIDATION;  // this library's bound: at most 8 quotient chunks (degree <= 9)
     if (log2u(prev) + pcs->log_blowup > 32) return ERR_INVALID;  // two-adicity of Goldilocks
+    const PcsParams fri{pcs->log_blowup, pcs->log_folding_arity, pcs->log_final_degree};
+    if (!fri_rounds_fit(fri, log2u(prev) + pcs->log_blowup)) return ERR_INVALID;  // no such last fold
     return OK;
 }
 }  // namespace p3g

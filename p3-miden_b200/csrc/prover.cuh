@@ -75,6 +75,18 @@ inline uint64_t inst_num_constraints(const Instance &I) {
     return I.air == AIR_SYMBOLIC ? I.sym->d.constraints.size() : air_num_constraints(I.air, I.width);
 }
 
+// FRI rounds: folds by 2^log_folding_arity until the degree is at most
+// 2^log_final_degree.
+inline uint64_t fri_rounds(const PcsParams &pcs, uint32_t log_lde) {
+    const uint32_t log_max_final = pcs.log_final_degree + pcs.log_blowup, log_a = pcs.log_folding_arity;
+    return log_lde > log_max_final ? (log_lde - log_max_final + log_a - 1) / log_a : 0;
+}
+// Whether the rounds fit the domain: with a blowup smaller than the arity the
+// last one may be larger than what is left to fold.
+inline bool fri_rounds_fit(const PcsParams &pcs, uint32_t log_lde) {
+    return fri_rounds(pcs, log_lde) * pcs.log_folding_arity <= log_lde;
+}
+
 struct Launcher {
     Ctx &ctx;
     uint64_t n = 0;
@@ -892,8 +904,7 @@ inline void prove(Ctx &ctx, const PcsParams &pcs, const Instance *inst, size_t n
     // ---- FRI commit phase
     const uint32_t log_a = pcs.log_folding_arity;
     const uint64_t arity = 1ull << log_a;
-    const uint32_t log_max_final = pcs.log_final_degree + lb;
-    const uint64_t rounds = log_lde > log_max_final ? (log_lde - log_max_final + log_a - 1) / log_a : 0;
+    const uint64_t rounds = fri_rounds(pcs, log_lde);
     const uint32_t log_final_size = log_lde - (uint32_t)rounds * log_a;
     const uint64_t final_deg = 1ull << (log_final_size > lb ? log_final_size - lb : 0);
     const uint64_t final_dom = final_deg << lb;

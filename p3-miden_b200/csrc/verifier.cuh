@@ -639,6 +639,10 @@ inline void prepare(const uint64_t *p2, const PcsParams &pcs, const Instance *in
     v.D = 1ull << v.log_qd;
     v.log_lde = v.log_max_h + lb;
     const uint32_t log_lde = v.log_lde;
+    if (!fri_rounds_fit(pcs, log_lde)) {
+        v.early = V_SHAPE;
+        return;
+    }
 
     // commitments and challenges in prover order
     uint64_t main_c[4], aux_c[4], quot_c[4];
@@ -683,8 +687,7 @@ inline void prepare(const uint64_t *p2, const PcsParams &pcs, const Instance *in
     // FRI oracle: round commitments, grinds, betas, final polynomial
     v.log_a = pcs.log_folding_arity;
     v.arity = 1ull << v.log_a;
-    const uint32_t log_max_final = pcs.log_final_degree + lb;
-    v.rounds = log_lde > log_max_final ? (log_lde - log_max_final + v.log_a - 1) / v.log_a : 0;
+    v.rounds = fri_rounds(pcs, log_lde);
     const uint32_t log_final_size = log_lde - (uint32_t)v.rounds * v.log_a;
     v.final_deg = 1ull << (log_final_size > lb ? log_final_size - lb : 0);
     std::vector<std::array<uint64_t, 4>> fri_c(v.rounds);
