@@ -224,7 +224,7 @@ __device__ __forceinline__ void p2_permute_dev(uint64_t *s) {
 
 // Permutation shared by 16 lanes, for latency-bound work (a few states at a
 // time; about 0.28 of the single-thread latency). Lane l < 12 holds word
-// l, lanes 12..15 hold zero between rounds. External rounds run one S-box per
+// l; what lanes 12..15 hold nobody reads. External rounds run one S-box per
 // lane and move the M4 and cross-block sums through shuffles. In the internal
 // rounds every lane carries a copy z of s_0: the S-box runs on z while the
 // sum R of s_1..s_11 is formed by a 4-step butterfly, and
