@@ -417,7 +417,7 @@ struct KArgs {
     // step; a base (a + b) - (c + c) whose two inner sums have no other reader
     // (the XOR of bits, a + b - 2ab) is emitted as (a - c) + (b - c).
     std::vector<uint32_t> n_users(n, 0);
-    std::vector<uint8_t> only_mul(n, 1), is_root(n, 0), weak(n, 0), fused(n, 0);
+    std::vector<uint8_t> only_mul(n, 1), is_root(n, 0), weak(n, 0), fused(n, 0), absorbed(n, 0);
     for (uint32_t c : d.constraints) is_root[c] = 1;
     for (size_t i = 0; i < n; i++) {
         const Node &x = d.nodes[i];
@@ -436,12 +436,14 @@ struct KArgs {
             const Node &sa = d.nodes[x.a], &sb = d.nodes[x.b];
             fused[i] = sa.op == ADD && sb.op == ADD && sb.a == sb.b && !A.ext[x.a] && !A.ext[x.b] &&
                        n_users[x.a] == 1 && n_users[x.b] == 1 && !is_root[x.a] && !is_root[x.b];
+            if (fused[i]) absorbed[x.a] = absorbed[x.b] = 1;
         }
     }
     // A third: a chain of sums and differences whose inner links each have one
     // reader, itself a link (such as the Horner recombination of a limb from
     // its bits, acc + acc + bit), is accumulated as a Wide and reduced once at
-    // the chain's end (inner[i]: i is such a link).
+    // the chain's end (inner[i]: i is such a link). The sums inside the form
+    // above are not emitted and read no Wide.
     std::vector<uint8_t> linear(n, 0), inner(n, 0);
     std::vector<int64_t> reader(n, -1);  // the one node reading i, -1 for none, -2 for several
     for (size_t i = 0; i < n; i++) {
@@ -452,7 +454,7 @@ struct KArgs {
         if (x.op == NEG) read(x.a);
     }
     for (size_t i = 0; i < n; i++)
-        inner[i] = linear[i] && !is_root[i] && reader[i] >= 0 && linear[reader[i]];
+        inner[i] = linear[i] && !is_root[i] && reader[i] >= 0 && linear[reader[i]] && !absorbed[reader[i]];
     std::vector<uint8_t> live(n);
     for (size_t c = c0; c < c1; c++) {
         const std::vector<ChunkGroup> &gs = A.chunks[c];
